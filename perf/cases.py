@@ -16,6 +16,7 @@ from mytrim_gb300 import Engine, LayerSpec, ElementSpec, _ffi as F, workloads as
 DATA = Path(W.__file__).resolve().parent / "data"
 COLL_PER_EV = 0.14
 VOXELS = 128
+ENERGIES = ("Eel", "Enuc", "Elost", "Eunfollowed", "Esputtered", "Evoxel", "eel_s2", "enuc_s2")
 
 # workload -> (beam energy [eV], mean elements per material, seconds per primary in FP32)
 RUNS = {
@@ -78,7 +79,7 @@ def draw(rng):
     if workload == "batched":
         return {"do": "run", "workload": workload, "precision": precision, "n": rng.randint(100, 4096),
                 "scale": round(math.exp(rng.uniform(math.log(0.002), math.log(0.01))), 5)}
-    most = 0.25 / (RUNS[workload][2] * SLOWER[precision])
+    most = (0.25 if precision == "fp32" else 0.1) / (RUNS[workload][2] * SLOWER[precision])
     case = {"do": "run", "workload": workload, "precision": precision, "n": _log_int(rng, max(64.0, most / 3000), most)}
     if workload == "arsenic" and precision == "fp32" and rng.random() < 0.5:
         case["log"] = True
@@ -132,17 +133,22 @@ def run(state):
     if case["do"] == "stopping":
         return e.stopping(case["Z"], case["m"], SIO2, state["energies"], precision=case["precision"])
     if case["do"] == "train":
-        rep = e.surrogate_train(n_train=case["n"], batch=case["batch"], epochs=case["epochs"], qat_epochs=case["qat"],
-                                seed=state["seed"] + 1, target="magic", weighting="transfer")
-        return {"loss": rep["final_loss"], "params": e.surrogate_params()}
+        e.surrogate_train(n_train=case["n"], batch=case["batch"], epochs=case["epochs"], qat_epochs=case["qat"],
+                          seed=state["seed"] + 1, target="magic", weighting="transfer")
+        return e.surrogate_params()
     res = e.run(state["sims"])
     if len(res) == 1:
         out = res[0]
     else:
         out = {k: np.concatenate([r[k].reshape(-1) for r in res]) if isinstance(v, np.ndarray)
                else np.array([r[k] for r in res]) for k, v in res[0].items()}
+    if case["precision"] != "fp64":
+        # these engines add energies in single precision first, lane by lane: two schedules of
+        # the same run (refill_min_idle 4 and 8, say) differ by up to 5e-9 in them, in nothing else
+        for k in ENERGIES:
+            out[k] = np.asarray(out[k], dtype=np.float32)
     if state["sims"][0].voxel_n[0]:
-        out["voxels"] = e.voxels(0, fp64=True)
+        out["voxels"] = e.voxels(0)
     if case.get("log"):
         ev = e.events()
         log = np.zeros(_log_slots(case), ev.dtype)  # the caller's table, as long as the log
@@ -166,7 +172,7 @@ def work(case):
                 "flops": 6 * 8512 * case["batch"] * steps + 128 * 60 * case["n"]}
     E, nel, _ = RUNS[case["workload"]]
     n = _primaries(case)
-    out = 8 * VOXELS ** 3 if case["workload"] == "gold" else 0
+    out = 4 * VOXELS ** 3 if case["workload"] == "gold" else 0
     return {"bytes": 60 * n + out, "flops": COLL_PER_EV * E * n * (300 + 91 * nel)}
 
 
@@ -351,7 +357,7 @@ def _train_exact(case, seed):
         at += m if k in scale else 0
     M, V = [torch.zeros_like(p) for p in P], [torch.zeros_like(p) for p in P]
     per = max(1, n // B)
-    total, loss = per * case["epochs"], 0.0
+    total = per * case["epochs"]
     rows = torch.arange(B, device=dev)
     for it in range(total):
         quant = it >= per * (case["epochs"] - case["qat"])
@@ -365,7 +371,6 @@ def _train_exact(case, seed):
             h.append(z[k] * torch.sigmoid(z[k]))
         d = h[3] @ P[6].T + P[7] - y
         wc = torch.stack([w, torch.full_like(w, 0.1)], 1)
-        loss = float((wc * d * d).sum() / B)
         g, dz = [None] * 8, 2 * wc * d / B
         for k in (3, 2, 1, 0):
             hid = k in (1, 2)
@@ -379,4 +384,4 @@ def _train_exact(case, seed):
             M[k] = 0.9 * M[k] + 0.1 * g[k]
             V[k] = 0.999 * V[k] + 0.001 * g[k] * g[k]
             P[k] = P[k] - lr * (M[k] / (1 - 0.9 ** t)) / (torch.sqrt(V[k] / (1 - 0.999 ** t)) + 1e-8)
-    return {"loss": loss, "params": torch.cat([p.reshape(-1) for p in P]).cpu().numpy()}
+    return torch.cat([p.reshape(-1) for p in P]).cpu().numpy()
