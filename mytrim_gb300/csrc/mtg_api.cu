@@ -77,14 +77,14 @@ struct mtg_ctx
   bool have_tables = false;
   mtg_config cfg;
   HostTables tables;
-  std::vector<Species32> sp32; // single-precision copies (FP32 engine), storage kept across batches
-  std::vector<Mat32> mc32;
+  std::vector<Mat32> mc32; // single-precision copies (FP32 engine), storage kept across batches
+  std::vector<MatCold32> cold32;
   std::vector<Sim32> sm32;
   bool prepared = false;
   bool launched = false;
   // device buffers
   DevBuf d_sims, d_prim_end, d_species, d_mats, d_row_species, d_stop;
-  DevBuf d_species32, d_mats32, d_sims32;
+  DevBuf d_mats32, d_cold32, d_sims32;
   DevBuf d_sg_params, d_sg_net; // surrogate network
   DevBuf d_vox, d_vox_range, d_vox_sum, d_vox_part; // energy-deposition voxels
   DevBuf d_cl, d_cl32, d_cl_next, d_cl_head, d_cl_mask; // sampleClusters geometry
@@ -187,9 +187,9 @@ setup_launch_shape(mtg_ctx * ctx)
     if (prec == MTG_PREC_FP64)
       tab = sizeof(SpeciesConst) * t.species.size() + sizeof(MatConst) * t.mats.size();
     else if (prec == MTG_PREC_FP32_SURROGATE)
-      tab = stage_net_offset(int(t.species.size()), int(t.mats.size())) + surrogate_net_bytes();
+      tab = stage_net_offset(int(t.mats.size())) + surrogate_net_bytes();
     else
-      tab = sizeof(Species32) * t.species.size() + sizeof(Mat32) * t.mats.size();
+      tab = sizeof(Mat32) * t.mats.size();
     if (tab <= 160 * 1024)
       ctx->stage = 1;
     else
@@ -209,7 +209,7 @@ setup_launch_shape(mtg_ctx * ctx)
   const int level = kernel_level(ctx);
   auto occupancy = [&](size_t smem, int * b) {
     return prec == MTG_PREC_FP64 ? occupancy64(ctx->block, smem, b, level)
-                                 : occupancy32(ctx->block, smem, b, prec == MTG_PREC_FP32_SURROGATE, level);
+                                 : occupancy32(ctx->block, smem, b, prec == MTG_PREC_FP32_SURROGATE, level, ctx->stage);
   };
   cudaError_t e = occupancy(ctx->smem, &bps);
   if (e != cudaSuccess)
@@ -262,12 +262,6 @@ fill_params(mtg_ctx * ctx, EngineParams & prm)
   {
     prm.species = ptr<SpeciesConst>(ctx->d_species);
     prm.mats = ptr<MatConst>(ctx->d_mats);
-  }
-  else
-  {
-    // the FP32 engine reads the single-precision copies through the same pointers
-    prm.species = reinterpret_cast<const SpeciesConst *>(ctx->d_species32.p);
-    prm.mats = reinterpret_cast<const MatConst *>(ctx->d_mats32.p);
   }
   prm.stage_tables = ctx->stage;
   prm.cold_offset = ctx->cold_offset;
@@ -379,6 +373,13 @@ launch_pass(mtg_ctx * ctx, int pass)
     ft.inv_dlnE = float(1.0 / ((std::log(ctx->tables.emax * 1.05) - std::log(STOP_EMIN)) / (STOP_N - 1)));
     ft.mlp = ctx->sg_ready ? ctx->d_sg_net.p : nullptr;
     ft.sims32 = ctx->d_sims32.p;
+    ft.mats32 = ctx->d_mats32.p;
+    ft.cold32 = ctx->d_cold32.p;
+    ft.cw = float(ctx->cfg.cw);
+    ft.tau = float(ctx->cfg.tau);
+    ft.flscale = float(1.0 / ctx->cfg.length_scale);
+    ft.one_sim = ctx->sm32.data();
+    ft.one_desc = ctx->sims_dev.data();
     e = launch_cascade32(prm, ft, ctx->grid, ctx->block, ctx->smem, ctx->stream,
                          prec == MTG_PREC_FP32_SURROGATE);
   }
@@ -478,7 +479,7 @@ mtg_destroy(mtg_ctx * ctx)
                      &ctx->d_ovf1,   &ctx->d_records,  &ctx->d_events,  &ctx->d_jobs,    &ctx->d_job_first,
                      &ctx->d_partials,
                      &ctx->d_out,    &ctx->d_tmp0,     &ctx->d_tmp1,    &ctx->d_tmp2,    &ctx->d_tmp3,
-                     &ctx->d_species32, &ctx->d_mats32, &ctx->d_sims32, &ctx->d_sg_params, &ctx->d_sg_net,
+                     &ctx->d_mats32, &ctx->d_cold32, &ctx->d_sims32, &ctx->d_sg_params, &ctx->d_sg_net,
                      &ctx->d_vox,    &ctx->d_vox_range, &ctx->d_vox_sum, &ctx->d_vox_part, &ctx->d_cl, &ctx->d_cl32,
                      &ctx->d_cl_next, &ctx->d_cl_head, &ctx->d_cl_mask};
   for (DevBuf * b : bufs)
@@ -652,10 +653,9 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
                                 int(nrows), d_row_species, ptr<float>(ctx->d_stop), lo, (hi - lo) / (STOP_N - 1),
                                 nullptr));
     CK(cudaDeviceSynchronize());
-    std::vector<Species32> & sp32 = ctx->sp32;
     std::vector<Mat32> & mc32 = ctx->mc32;
     std::vector<Sim32> & sm32 = ctx->sm32;
-    build_fp32_tables(t, sp32, mc32, sm32);
+    build_fp32_tables(t, mc32, ctx->cold32, sm32);
     if (!t.clusters.empty() || !t.cl_head.empty())
     {
       std::vector<Cl4f> c32(t.clusters.size());
@@ -674,11 +674,11 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
           sm32[i].cl_mask = ptr<uint32_t>(ctx->d_cl_mask) + t.sims[i].mask_base;
         }
     }
-    CK(ensure(ctx->d_species32, sizeof(Species32) * sp32.size()));
     CK(ensure(ctx->d_mats32, sizeof(Mat32) * mc32.size()));
+    CK(ensure(ctx->d_cold32, sizeof(MatCold32) * ctx->cold32.size()));
     CK(ensure(ctx->d_sims32, sizeof(Sim32) * sm32.size()));
-    CK(h2d(ctx, ctx->d_species32.p, sp32.data(), sizeof(Species32) * sp32.size()));
     CK(h2d(ctx, ctx->d_mats32.p, mc32.data(), sizeof(Mat32) * mc32.size()));
+    CK(h2d(ctx, ctx->d_cold32.p, ctx->cold32.data(), sizeof(MatCold32) * ctx->cold32.size()));
     CK(h2d(ctx, ctx->d_sims32.p, sm32.data(), sizeof(Sim32) * sm32.size()));
   }
   if (ctx->record_cap > 0)
@@ -915,7 +915,7 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
                      &ctx->d_hist,   &ctx->d_err,      &ctx->d_counters, &ctx->d_stacks, &ctx->d_ovf0,
                      &ctx->d_ovf1,   &ctx->d_records,  &ctx->d_events,  &ctx->d_jobs,    &ctx->d_job_first,
                      &ctx->d_partials,
-                     &ctx->d_out,    &ctx->d_species32, &ctx->d_mats32, &ctx->d_sims32, &ctx->d_vox, &ctx->d_vox_part};
+                     &ctx->d_out,    &ctx->d_mats32, &ctx->d_cold32, &ctx->d_sims32, &ctx->d_vox, &ctx->d_vox_part};
   for (DevBuf * b : bufs)
     bytes += b->bytes;
   ctx->stats.device_bytes = bytes;

@@ -158,8 +158,8 @@ widen_f32(float f)
 }
 
 // Plain FP32 accumulator for the per-collision energy sums of the FP32 engine;
-// the engine hands it to the FP64 per-primary arrays every few dozen collisions
-// (Pol::FLUSH_EVERY), so each float sum stays short and accurate to ~1e-7
+// the engine hands it to the FP64 per-primary arrays every 64 collisions
+// (LaneSink::hand_over), so each float sum stays short and accurate to ~1e-7
 struct AccF32
 {
   float s;
@@ -201,7 +201,8 @@ struct AccKahan32
 template <class Acc>
 struct LaneCold
 {
-  unsigned int n_repl, n_inter, n_subst, n_lost, n_members, n_passes, n_fallbacks, n_sput, n_back;
+  unsigned int n_rest[4]; // members come to rest, by state; each replacement or substitution is one replacement event
+  unsigned int n_lost, n_members, n_passes, n_fallbacks, n_sput, n_back;
   unsigned int m_vac;
   int m_state;
   unsigned int n_dropped; // depth-histogram events beyond the last bin
@@ -255,6 +256,28 @@ level_events(int lvl)
   return lvl == LVL_EVENTS || lvl == LVL_FULL || lvl == LVL_CLU_EV;
 }
 
+// the single-precision kernel's tallies (mtg_cascade32.cuh)
+struct Sink32
+{
+  using Acc = AccKahan32;
+  using AccHot = AccF32;
+  using Real = float;
+};
+
+// generation and species of a member (a kernel that packs them overloads these)
+template <class P>
+__device__ __forceinline__ int
+member_gen(const P & p)
+{
+  return p.gen;
+}
+template <class P>
+__device__ __forceinline__ int
+member_species(const P & p)
+{
+  return p.species;
+}
+
 // Device tally sink for one lane of a kernel of level LVL.
 template <class Pol, int LVL>
 struct LaneSink
@@ -266,7 +289,9 @@ struct LaneSink
   using Real = typename Pol::Real;
   LaneCold<Acc> * cold;
   const EngineParams * prm;
+  unsigned int * s_hist; // the block's vacancy and replacement counters (prm->hist_smem_bins of them)
   const SimDesc * sim;
+  int isim;            // its index
   long long gprim;     // global primary index of the current member
   int range_mode;
   // per-primary accumulators
@@ -282,7 +307,8 @@ struct LaneSink
   __device__ void reset_sim()
   {
     LaneCold<Acc> & c = *cold;
-    c.n_repl = c.n_inter = c.n_subst = c.n_lost = c.n_members = c.n_passes = c.n_fallbacks = 0;
+    c.n_rest[ST_REPLACEMENT] = c.n_rest[ST_SUBSTITUTIONAL] = c.n_rest[ST_INTERSTITIAL] = 0;
+    c.n_lost = c.n_members = c.n_passes = c.n_fallbacks = 0;
     c.n_sput = c.n_back = c.n_dropped = 0;
     n_newton = 0;
     c.e_lost.reset();
@@ -352,7 +378,7 @@ struct LaneSink
     r.aux = double(aux);
     r.key = key;
     r.primary = gprim - sim->prim_begin + sim->key_offset;
-    r.sim = int(sim - prm->sims);
+    r.sim = isim;
     r.kind = kind;
     r.Z = Z;
     r.m = double(m);
@@ -367,8 +393,8 @@ struct LaneSink
   __device__ void history(const P & p, int Z1, Real m1)
   {
     if constexpr (EV)
-      event(EV_HISTORY, Real(p.x), Real(p.y), Real(p.z), Real(p.E), Z1, m1, p.gen, 0, Real(0), p.key, p.tag,
-            cold->m_md);
+      event(EV_HISTORY, Real(p.x), Real(p.y), Real(p.z), Real(p.E), Z1, m1, member_gen(p), 0, Real(0), p.key,
+            p.tag, cold->m_md);
   }
   // followRecoil (trim.C:362): a displaced recoil, followed or not
   template <class R, class E>
@@ -458,15 +484,15 @@ struct LaneSink
   {
     LaneCold<Acc> & c = *cold;
     if constexpr (EV)
-      event(EV_LOST, Real(p.x), Real(p.y), Real(p.z), Real(p.E), Z1, m1, p.gen, ST_LOST, e - Real(p.E), p.key, p.tag,
-            cold->m_md);
+      event(EV_LOST, Real(p.x), Real(p.y), Real(p.z), Real(p.E), Z1, m1, member_gen(p), ST_LOST, e - Real(p.E),
+            p.key, p.tag, cold->m_md);
     ++c.n_lost;
     c.e_lost.add(e);
     if (MID && prm->records)
       c.m_state = ST_LOST;
     if (p.x < Real(0) && sim->bc[0] == 2)
     {
-      if (p.gen == 0)
+      if (member_gen(p) == 0)
         ++c.n_back;
       else if (sim->surface_binding > 0.0f && Real(p.E) * p.dx * p.dx > Real(sim->surface_binding))
       {
@@ -477,11 +503,93 @@ struct LaneSink
   }
 
   template <class R, class E>
-  __device__ void vacancy(const R & rec, const E & el, Real Erec, uint64_t key)
+  __device__ void vacancy_event(const R & rec, const E & el, Real Erec, uint64_t key)
   {
     if constexpr (EV)
       event(EV_VACANCY, Real(rec.x), Real(rec.y), Real(rec.z), Erec, el.Z2, Real(el.m2), rec.gen, 0,
             Real(el.Elbind), key, rec.tag);
+  }
+  template <class R, class E>
+  __device__ void replacement_event(const R & rec, const E & el, Real Erec, uint64_t key)
+  {
+    if constexpr (EV)
+      event(EV_REPLACEMENT, Real(rec.x), Real(rec.y), Real(rec.z), Erec, el.Z2, Real(el.m2), rec.gen, 0,
+            Real(el.Elbind), key, rec.tag);
+  }
+  // vacancies by the member that makes them, for the member records
+  __device__ void member_vacancy(unsigned int add)
+  {
+    if (MID && prm->records)
+      cold->m_vac += add;
+  }
+  // a displaced recoil as its followed member starts (single-precision kernel): the
+  // vacancy or the replacement that the collision left behind
+  __device__ void displaced(bool vac, Real x, Real Erec)
+  {
+    if (vac)
+    {
+      ++a_vac;
+      if (MID && range_mode)
+        return;
+      vacancy_bins(x, Erec);
+    }
+    else
+      replacement_bin(x);
+    count_bins();
+  }
+  // the depth histograms' counts of the vacancy or replacement just binned
+  __device__ void count_bins()
+  {
+    const int hb = vac_bin >= 0 ? vac_bin : repl_bin;
+    if (hb >= 0)
+    {
+      if (prm->hist_smem_bins)
+        atomicAdd(s_hist + (hb - prm->hist_smem_base), 1u);
+      else
+        atomicAdd(prm->hist + hb, 1ull);
+    }
+    vac_bin = repl_bin = -1;
+    if (MID && prm->any_evac)
+    {
+      if (cold->evac_bin >= 0)
+        atomicAdd(prm->hist + cold->evac_bin, 1ull);
+      cold->evac_bin = -1;
+    }
+  }
+  __device__ void vacancy_bins(Real x, Real Erec)
+  {
+    const int b = depth_bin(x, inv_vac_bin(), sim->hist_vac_n);
+    if (b >= 0)
+    {
+      vac_bin = int(sim->hist_vac_base) + b;
+      if (MID && prm->any_evac && sim->hist_evac_rows > 0)
+      {
+        // TrimVacEnergyCount::vacancyCreation (apps/src/TrimVacEnergyCount.C:32-53):
+        // row int(ln E) of the recoil energy, negative rows in row 0
+        int row = int(loge(Erec));
+        row = row < 0 ? 0 : row;
+        if (row < sim->hist_evac_rows)
+          cold->evac_bin = int(sim->hist_evac_base) + row * sim->hist_vac_n + b;
+        else
+          ++cold->n_dropped;
+      }
+    }
+    else if (b == BIN_BEYOND)
+      ++cold->n_dropped;
+  }
+  __device__ void replacement_bin(Real x)
+  {
+    const int b = depth_bin(x, inv_vac_bin(), sim->hist_vac_n);
+    if (b >= 0)
+      repl_bin = int(sim->hist_vac_base + sim->hist_vac_n) + b;
+    else if (b == BIN_BEYOND)
+      ++cold->n_dropped;
+  }
+
+  // vacancyCreation's tally (its event: vacancy_event)
+  template <class R, class E>
+  __device__ void vacancy(const R & rec, const E & el, Real Erec)
+  {
     if (MID && range_mode == 2)
     {
       // TrimPrimaries::vacancyCreation (trim.C:446-464): one vacancy per displaced
@@ -498,8 +606,7 @@ struct LaneSink
         add += (unsigned int)(int(Real(0.8) * Ev / (Real(2) * Real(el.Edisp))));
       }
       a_vac += add;
-      if (prm->records)
-        cold->m_vac += add;
+      member_vacancy(add);
       return;
     }
     if (MID && range_mode)
@@ -521,60 +628,44 @@ struct LaneSink
       else
         add = 1;
       a_vac += add;
-      if (prm->records)
-        cold->m_vac += add;
+      member_vacancy(add);
       return;
     }
     ++a_vac;
-    if (MID && prm->records)
-      ++cold->m_vac;
-    const int b = depth_bin(Real(rec.x), inv_vac_bin(), sim->hist_vac_n);
-    if (b >= 0)
-    {
-      vac_bin = int(sim->hist_vac_base) + b;
-      if (MID && prm->any_evac && sim->hist_evac_rows > 0)
-      {
-        // TrimVacEnergyCount::vacancyCreation (apps/src/TrimVacEnergyCount.C:32-53):
-        // row int(ln E) of the recoil energy, negative rows in row 0
-        int row = int(loge(Erec));
-        row = row < 0 ? 0 : row;
-        if (row < sim->hist_evac_rows)
-          cold->evac_bin = int(sim->hist_evac_base) + row * sim->hist_vac_n + b;
-        else
-          ++cold->n_dropped;
-      }
-    }
-    else if (b == BIN_BEYOND)
-      ++cold->n_dropped;
+    member_vacancy(1u);
+    vacancy_bins(Real(rec.x), Erec);
+  }
+  // replacementCollision's tally
+  template <class R>
+  __device__ void replacement(const R & rec)
+  {
+    replacement_bin(Real(rec.x));
+  }
+  // event and tally
+  template <class R, class E>
+  __device__ void vacancy(const R & rec, const E & el, Real Erec, uint64_t key)
+  {
+    vacancy_event(rec, el, Erec, key);
+    vacancy(rec, el, Erec);
   }
   template <class R, class E>
   __device__ void replacement(const R & rec, const E & el, Real Erec, uint64_t key)
   {
-    if constexpr (EV)
-      event(EV_REPLACEMENT, Real(rec.x), Real(rec.y), Real(rec.z), Erec, el.Z2, Real(el.m2), rec.gen, 0,
-            Real(el.Elbind), key, rec.tag);
-    ++cold->n_repl;
-    const int b = depth_bin(Real(rec.x), inv_vac_bin(), sim->hist_vac_n);
-    if (b >= 0)
-      repl_bin = int(sim->hist_vac_base + sim->hist_vac_n) + b;
-    else if (b == BIN_BEYOND)
-      ++cold->n_dropped;
+    replacement_event(rec, el, Erec, key);
+    replacement(rec);
   }
   template <class P>
   __device__ void stop(int state, const P & p, int Z1, Real m1)
   {
     if constexpr (EV)
-      event(EV_REST, Real(p.x), Real(p.y), Real(p.z), Real(p.E), Z1, m1, p.gen, state, Real(0), p.key, p.tag,
-            cold->m_md);
+      event(EV_REST, Real(p.x), Real(p.y), Real(p.z), Real(p.E), Z1, m1, member_gen(p), state, Real(0), p.key,
+            p.tag, cold->m_md);
     if (MID && prm->records)
       cold->m_state = state;
     a_enuc.add(Real(p.E));
     deposit(Real(p.x), Real(p.y), Real(p.z), Real(p.E));
-    if (state == ST_INTERSTITIAL)
-      ++cold->n_inter;
-    else if (state == ST_SUBSTITUTIONAL)
-      ++cold->n_subst;
-    if (p.gen == 0)
+    ++cold->n_rest[state];
+    if (member_gen(p) == 0)
     {
       prm->prim.fx[gprim] = double(p.x);
       prm->prim.fy[gprim] = double(p.y);
@@ -636,20 +727,38 @@ struct LaneSink
       return pow64(x, y);
   }
 
-  // every Pol::FLUSH_EVERY collisions of a lane, hand the energy sums to the
-  // per-primary arrays (no-op for FLUSH_EVERY = 0)
-  __device__ void tick()
+  // hand the energy sums to the per-primary arrays: the single-precision kernel does it
+  // on every 64th iteration, so that its sums stay short
+  __device__ void hand_over()
   {
-    if constexpr (Pol::FLUSH_EVERY > 0)
-      if ((a_coll & unsigned(Pol::FLUSH_EVERY - 1)) == 0u)
-      {
-        if (a_eel.nonzero())
-          a_eel.atomic_add_to(prm->prim.eel + gprim);
-        if (a_enuc.nonzero())
-          a_enuc.atomic_add_to(prm->prim.enuc + gprim);
-        a_eel.reset();
-        a_enuc.reset();
-      }
+    if (a_eel.nonzero())
+      a_eel.atomic_add_to(prm->prim.eel + gprim);
+    if (a_enuc.nonzero())
+      a_enuc.atomic_add_to(prm->prim.enuc + gprim);
+    a_eel.reset();
+    a_enuc.reset();
+  }
+  // the record of a member that has ended (records runs)
+  template <class P>
+  __device__ void record(const P & p, unsigned int ncoll)
+  {
+    const unsigned long long slot = atomicAdd(prm->n_records, 1ull);
+    if ((long long)slot >= prm->records_cap)
+      return;
+    MemberRecord m;
+    m.key = p.key;
+    m.sim = p.sim;
+    m.species = member_species(p);
+    m.gen = member_gen(p);
+    m.state = cold->m_state;
+    m.ncoll = ncoll;
+    m.nvac = cold->m_vac;
+    m.E = double(p.E);
+    m.x = double(p.x);
+    m.y = double(p.y);
+    m.z = double(p.z);
+    m.eel = cold->m_eel.value();
+    prm->records[slot] = m;
   }
 
   __device__ void flush_prim()
@@ -675,12 +784,12 @@ struct LaneSink
     using ull = unsigned long long;
     if (c.n_members)
       atomicAdd(&t->members, ull(c.n_members));
-    if (c.n_repl)
-      atomicAdd(&t->replacements, ull(c.n_repl));
-    if (c.n_inter)
-      atomicAdd(&t->interstitials, ull(c.n_inter));
-    if (c.n_subst)
-      atomicAdd(&t->substitutionals, ull(c.n_subst));
+    if (const unsigned int n = c.n_rest[ST_REPLACEMENT] + c.n_rest[ST_SUBSTITUTIONAL])
+      atomicAdd(&t->replacements, ull(n));
+    if (c.n_rest[ST_INTERSTITIAL])
+      atomicAdd(&t->interstitials, ull(c.n_rest[ST_INTERSTITIAL]));
+    if (c.n_rest[ST_SUBSTITUTIONAL])
+      atomicAdd(&t->substitutionals, ull(c.n_rest[ST_SUBSTITUTIONAL]));
     if (c.n_lost)
       atomicAdd(&t->lost, ull(c.n_lost));
     if (n_newton)
@@ -767,6 +876,8 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
   sink.cold->evac_bin = -1;
   sink.cold->ev_next = sink.cold->ev_end = 0;
   sink.prm = &prm;
+  sink.s_hist = s_hist;
+  sink.vac_bin = sink.repl_bin = -1;
   sink.sim = nullptr;
   sink.gprim = -1;
   sink.range_mode = 0;
@@ -786,6 +897,7 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
       cur_sim = p.sim;
       sim = prm.sims + cur_sim;
       sink.sim = sim;
+      sink.isim = cur_sim;
       sink.range_mode = sim->range_mode;
       sink.vox = MID && prm.voxels != nullptr && sim->voxel_n[0] > 0;
       sink.gprim = -1;
@@ -802,11 +914,7 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
     {
       // IonMDTag: the demo programs' MD-gap mark, taken when the member starts
       // (apps/mytrim_solid.C:156-159); a spawned recoil's _md is 0 (ion.C:88-93)
-      bool gap;
-      if constexpr (sizeof(typename Pol::Real) == 8)
-        gap = double(p.E) > sim->md_Emin && double(p.E) < sim->md_Emax;
-      else
-        gap = float(p.E) > sim->md_Emin_f && float(p.E) < sim->md_Emax_f; // no FP64 in the FP32 engine
+      const bool gap = double(p.E) > sim->md_Emin && double(p.E) < sim->md_Emax;
       sink.cold->m_md = (sim->md_Z != 0 && mctx.sc->Z1 == sim->md_Z && gap) ? 1 : 0;
     }
     r1 = Pol::first_draw(p.key, prm.k0, prm.k1);
@@ -868,8 +976,6 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
     // ---- one collision per live lane
     Particle rec;
     int flags = 0;
-    sink.vac_bin = -1;
-    sink.repl_bin = -1;
     if (live)
     {
       ++ic;
@@ -882,7 +988,6 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
     {
       if (flags & CF_VOID)
         --sink.a_coll; // the member left without a collision (no checkPKAState)
-      sink.tick();
       if (!(flags & CF_DONE) && ic >= prm.max_collisions)
       {
         atomicOr(prm.error_flags, ERRB_BUDGET);
@@ -892,26 +997,7 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
       {
         live = false;
         if (MID && prm.records)
-        {
-          const unsigned long long slot = atomicAdd(prm.n_records, 1ull);
-          if ((long long)slot < prm.records_cap)
-          {
-            MemberRecord m;
-            m.key = p.key;
-            m.sim = p.sim;
-            m.species = p.species;
-            m.gen = p.gen;
-            m.state = sink.cold->m_state;
-            m.ncoll = ic;
-            m.nvac = sink.cold->m_vac;
-            m.E = double(p.E);
-            m.x = double(p.x);
-            m.y = double(p.y);
-            m.z = double(p.z);
-            m.eel = sink.cold->m_eel.value();
-            prm.records[slot] = m;
-          }
-        }
+          sink.record(p, ic);
       }
       if (flags & CF_PUSH)
       {
@@ -922,22 +1008,7 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
     // depth histograms: a collision makes a vacancy or a replacement, never both;
     // about one lane in ten has an event, so each adds its own count (aggregating
     // lanes with __match_any_sync cost more than it saved)
-    {
-      const int hb = sink.vac_bin >= 0 ? sink.vac_bin : sink.repl_bin;
-      if (hb >= 0)
-      {
-        if (prm.hist_smem_bins)
-          atomicAdd(s_hist + (hb - prm.hist_smem_base), 1u);
-        else
-          atomicAdd(prm.hist + hb, 1ull);
-      }
-    }
-    if (MID && prm.any_evac)
-    {
-      if (sink.cold->evac_bin >= 0)
-        atomicAdd(prm.hist + sink.cold->evac_bin, 1ull);
-      sink.cold->evac_bin = -1;
-    }
+    sink.count_bins();
 
     // ---- push displaced recoils onto the warp stack
     const bool push = (flags & CF_PUSH) != 0;

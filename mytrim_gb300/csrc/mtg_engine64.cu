@@ -20,7 +20,6 @@ struct Fp64Policy
   using Real = double;
   using Acc = AccF64;
   using AccHot = AccF64;
-  static constexpr int FLUSH_EVERY = 0;
   static constexpr int min_blocks(int) { return MTG_FP64_MIN_BLOCKS; } // 3: <= 170 registers, 12 warps per SM
 
   struct Tables

@@ -31,13 +31,18 @@ struct Fp32Tables
   float inv_dlnE;       // 1 / spacing in ln E
   const void * mlp;     // surrogate weights, NULL without the surrogate
   const void * sims32;  // Sim32 per simulation
+  const void * mats32;  // Mat32 and MatCold32 rows
+  const void * cold32;
+  float cw, tau, flscale; // run-wide settings: first-flight cap, tau, 1 / length scale
+  const Sim32 * one_sim;  // host copies of a single-simulation run's constants, its device
+  const SimDesc * one_desc; // pointers patched in
 };
 cudaError_t launch_build_stop_tables(const SpeciesConst * species, const MatConst * mats, const int * row_mat,
                                      int n_rows, const int * row_species, float * out, double lnE_min,
                                      double dlnE, cudaStream_t st);
 cudaError_t launch_cascade32(const EngineParams & prm, const Fp32Tables & t, int grid, int block, size_t smem,
                              cudaStream_t st, int surrogate);
-cudaError_t occupancy32(int block, size_t smem, int * blocks_per_sm, int surrogate, int level);
+cudaError_t occupancy32(int block, size_t smem, int * blocks_per_sm, int surrogate, int level, int one);
 size_t record_size32();
 size_t cold_slot_bytes32();
 cudaError_t launch_scatter32(const double * eps, const double * b, long long n, double * s2, int potential,

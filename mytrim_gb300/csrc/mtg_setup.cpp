@@ -213,48 +213,50 @@ patch_cluster_pointers(std::vector<SimDesc> & sims, const Cl4d * cl, const int *
 }
 
 void
-build_fp32_tables(const HostTables & t, std::vector<Species32> & species, std::vector<Mat32> & mats,
+build_fp32_tables(const HostTables & t, std::vector<Mat32> & mats, std::vector<MatCold32> & cold,
                   std::vector<Sim32> & sims)
 {
-  species.resize(t.species.size());
-  for (size_t i = 0; i < t.species.size(); ++i)
-  {
-    std::memset(&species[i], 0, sizeof(Species32));
-    species[i].m1 = float(t.species[i].m1);
-    species[i].two_m1 = float(2.0 * t.species[i].m1);
-    species[i].Z1 = t.species[i].Z1;
-  }
   mats.resize(t.mats.size());
-  for (size_t i = 0; i < t.mats.size(); ++i)
-  {
-    const MatConst & m = t.mats[i];
-    Mat32 & o = mats[i];
-    std::memset(&o, 0, sizeof o);
-    o.a = float(m.a);
-    o.f = float(m.f);
-    o.epsdg = float(m.epsdg);
-    o.inv_pi_arho = float(1.0 / (3.14159265358979323846 * m.arho));
-    o.nel = m.nel;
-    o.row = m.row;
-    for (int j = 0; j < m.nel; ++j)
-    {
-      const ElemConst & e = m.el[j];
-      Elem32 & f = o.el[j];
-      f.t = float(e.t);
-      f.my = float(e.my);
-      f.ec = float(e.ec);
-      f.inv_ai = float(1.0 / e.ai);
-      f.fi = float(e.fi);
-      f.Edisp = float(e.Edisp);
-      f.Elbind = float(e.Elbind);
-      f.m2 = float(e.m2);
-      f.disp_thresh = float(e.Edisp - e.Elbind);
-      f.maz = float(e.maz);
-      f.mam = float(e.mam);
-      f.Z2 = e.Z2;
-      f.rspecies = e.rspecies;
-    }
-  }
+  cold.resize(t.mats.size());
+  for (const SimDesc & d : t.sims)
+    for (int sp = 0; sp < d.n_species; ++sp)
+      for (int k = 0; k < d.n_mat; ++k)
+      {
+        const size_t i = size_t(d.mat_base) + size_t(sp) * d.n_mat + k;
+        const SpeciesConst & sc = t.species[size_t(d.species_base) + sp];
+        const MatConst & m = t.mats[i];
+        Mat32 & o = mats[i];
+        MatCold32 & c = cold[i];
+        std::memset(&o, 0, sizeof o);
+        std::memset(&c, 0, sizeof c);
+        o.two_m1 = float(2.0 * sc.m1);
+        o.a = float(m.a);
+        o.f = float(m.f);
+        o.epsdg = float(m.epsdg);
+        o.inv_pi_arho = float(1.0 / (3.14159265358979323846 * m.arho));
+        o.nel = m.nel;
+        o.row = m.row;
+        c.m1 = float(sc.m1);
+        c.Z1 = sc.Z1;
+        c.maz = float(m.az);
+        c.mam = float(m.am);
+        for (int j = 0; j < m.nel; ++j)
+        {
+          const ElemConst & e = m.el[j];
+          Elem32 & f = o.el[j];
+          o.t[j] = float(e.t);
+          f.my = float(e.my);
+          f.ec = float(e.ec);
+          f.inv_ai = float(1.0 / e.ai);
+          f.fi = float(e.fi);
+          f.Edisp = float(e.Edisp);
+          f.Elbind = float(e.Elbind);
+          f.disp_thresh = float(e.Edisp - e.Elbind);
+          f.recoil = e.rspecies | (sc.Z1 == e.Z2 ? ST_REPLACEMENT : ST_SUBSTITUTIONAL) << 8;
+          c.Z2[j] = e.Z2;
+          c.m2[j] = float(e.m2);
+        }
+      }
   sims.resize(t.sims.size());
   for (size_t i = 0; i < t.sims.size(); ++i)
   {

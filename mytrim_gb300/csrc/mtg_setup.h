@@ -58,7 +58,7 @@ int make_material(const mtg_scoef_row * rows, const SpeciesConst & sc, const mtg
                   double tmin, MatConst & out, std::string & err);
 
 // Single-precision copies of the tables for the FP32 engine.
-void build_fp32_tables(const HostTables & t, std::vector<Species32> & species, std::vector<Mat32> & mats,
+void build_fp32_tables(const HostTables & t, std::vector<Mat32> & mats, std::vector<MatCold32> & cold,
                        std::vector<Sim32> & sims);
 
 // Philox key of a run seed

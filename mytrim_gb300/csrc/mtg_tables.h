@@ -196,36 +196,41 @@ enum EventKind : int
 };
 
 // ---- single-precision copies used by the FP32 engine (built from the tables above)
-struct Elem32
+// Rows are read in 16-byte pieces; what the collision loop does not read is in MatCold32.
+struct alignas(16) Elem32
 {
-  float t, my, ec, inv_ai, fi, Edisp, Elbind, m2;
-  float disp_thresh; // Edisp - Elbind (trim.C:359)
-  float maz, mam;    // material mean Z and mass (TrimPrimaries)
-  int Z2, rspecies;
+  float fi, inv_ai, ec, my;
+  float Elbind, disp_thresh, Edisp; // disp_thresh = Edisp - Elbind (trim.C:359)
+  int recoil; // species of a recoil, and << 8 what a projectile that takes its place has come to rest as
 };
 
-struct Mat32
+struct alignas(16) Mat32
 {
-  float a, f, epsdg, inv_pi_arho; // 1 / (pi * atomic density)
-  int nel, row, pad0, pad1;       // row: stopping-table row of this (species, material)
+  float inv_pi_arho, two_m1; // 1 / (pi * atomic density), twice the projectile's mass
+  int row, nel;              // stopping-table row of this (species, material)
+  float t[MAX_EL];
+  float a, f, epsdg, pad;
   Elem32 el[MAX_EL];
 };
 
-struct Species32
+struct MatCold32
 {
-  float m1, two_m1;
-  int Z1, pad;
+  float m1;
+  int Z1;
+  float maz, mam; // material mean Z and mass (TrimPrimaries)
+  int Z2[MAX_EL];
+  float m2[MAX_EL];
 };
 
 // byte offset of the surrogate network in the FP32 engine's staged shared-memory
-// tables: after the species and material rows, 16-byte aligned
+// tables: after the material rows
 #ifdef __CUDACC__
 __host__ __device__
 #endif
 inline size_t
-stage_net_offset(int n_species, int n_mats)
+stage_net_offset(int n_mats)
 {
-  return (sizeof(Species32) * size_t(n_species) + sizeof(Mat32) * size_t(n_mats) + 15) / 16 * 16;
+  return sizeof(Mat32) * size_t(n_mats);
 }
 
 struct Sim32
