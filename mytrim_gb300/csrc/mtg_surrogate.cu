@@ -12,14 +12,15 @@
 //   [0, 12] (b = 12 sqrt(U)), drawn from Philox.  The sin^2(theta/2) target is the
 //   quadrature's or, on request, the FP64 magic formula's at the same samples
 //   (scatter64: the reference's Newton solve and magic formula, trim.C:180-271).
-// * Training: the project's own FP32 kernels -- dense forward, backward (data and
-//   weight gradients, deterministic two-stage reduction), MSE loss, Adam -- with the
-//   whole step captured in a CUDA graph.  The last epochs are quantisation-aware:
+// * Training: the project's own FP32 kernels, two a step: forward and backward pass
+//   (the blocks' weight gradients added in block order, so that a run repeats bit for
+//   bit) and Adam.  The last epochs are quantisation-aware:
 //   the two hidden 64x64 layers see BF16-rounded weights and inputs in the forward
 //   pass, as in inference.
 // * Inference: mtg_surrogate.cuh.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -180,171 +181,355 @@ bf16_round(float v)
   return __bfloat162float(__float2bfloat16_rn(v));
 }
 
-__device__ __forceinline__ float
-silu_d(float z)
+// ---- one training step
+//
+// A batch step is 25,000 multiply-adds a sample (forward, data gradients, weight
+// gradients) on weights that fit a corner of shared memory, so the whole step is one
+// kernel: a block takes 64 samples through all layers and back without leaving the SM,
+// and keeps the weight gradients of its samples in registers (4 x 4 of each 64 x 64
+// layer per thread) until it has done all its tiles.  A second kernel adds the blocks'
+// gradients in block order (at most one block per SM) and takes the Adam step.  Layer by
+// layer through global memory, with a thread per output, a step of 16,384 samples took
+// 0.68 ms (64 steps with their 131,072 samples' targets 50.6 ms, now 9.6); it is FP32 throughout, each sum in the same order as then but for the weight
+// gradients' grouping by block.
+//
+// The 64 x 64 products read their operands from rows of 68 floats: a warp's 16-byte reads
+// along a row, and of one column of 16 rows, then fall on different banks.
+constexpr int TS = 64; // samples per tile
+constexpr int TLD = 68;
+struct TrainSmem
+{
+  float w1[SG_H * 2], b1[SG_H], b2[SG_H], b3[SG_H], w4[2 * SG_H], b4[2], pad[2];
+  float w2[SG_H][TLD], w3[SG_H][TLD]; // [out][in]
+  float h[3][TS][TLD];                // layer outputs
+  float d[3][TS][TLD];                // silu'(z), then the gradient of z
+  float x[TS][2], y[TS][2], wt[TS], dO[TS][2];
+  float red[4][SG_H];
+};
+
+// z -> silu(z), silu'(z)
+__device__ __forceinline__ void
+silu_pair(float z, float & h, float & dh)
 {
   const float s = 1.0f / (1.0f + expf(-z));
-  return s * (1.0f + z * (1.0f - s));
+  h = z * s;
+  dh = s * (1.0f + z * (1.0f - s));
 }
 
-__device__ __forceinline__ float
-silu_acc(float z)
+// h_out = silu(h_in W^T + b) and its derivative, for the tile's 64 x 64 outputs; thread
+// (ts, tn) does samples 4 ts .. 4 ts + 3 and outputs tn, tn + 16, tn + 32, tn + 48
+__device__ __forceinline__ void
+tile_forward(const float (*in)[TLD], const float (*w)[TLD], const float * bias, float (*out)[TLD], float (*der)[TLD],
+             bool round_out)
 {
-  return z / (1.0f + expf(-z));
-}
-
-// Z = X W^T + b, H = silu(Z) (act) or Z; X [B][K], W [N][K]; one thread per (sample, output)
-__global__ void
-dense_fwd(const float * X, int K, const float * W, const float * bias, int N, long long B, float * Z, float * H,
-          int act, int quant)
-{
-  extern __shared__ float sw[]; // W [N][K]
-  for (int i = threadIdx.x; i < N * K; i += blockDim.x)
-    sw[i] = quant ? bf16_round(W[i]) : W[i];
-  __syncthreads();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= B * N)
-    return;
-  const long long s = idx / N;
-  const int n = int(idx % N);
-  float z = bias[n];
-  const float * xr = X + s * K;
-  for (int k = 0; k < K; ++k)
-    z = fmaf(quant ? bf16_round(xr[k]) : xr[k], sw[n * K + k], z);
-  Z[idx] = z;
-  if (H)
-    H[idx] = act ? silu_acc(z) : z;
-}
-
-// loss and output gradient: dO = 2 w_c (O - Y) / B; output 0 weighted per sample
-// by W (NULL: 1), output 1 by w1
-__global__ void
-loss_grad(const float * O, const float * Y, const float * W, long long B, float w1, float * dO, float * loss_partial)
-{
-  __shared__ float red[256];
-  float acc = 0.0f;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < B * 2; i += (long long)gridDim.x * blockDim.x)
+  const int ts = threadIdx.x >> 4, tn = threadIdx.x & 15;
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      acc[i][j] = bias[tn + 16 * j];
+#pragma unroll 4
+  for (int k = 0; k < SG_H; k += 4)
   {
-    const float wc = (i & 1) ? w1 : (W ? W[i >> 1] : 1.0f);
-    const float d = O[i] - Y[i];
-    dO[i] = 2.0f * wc * d / float(B);
-    acc += wc * d * d;
+    float4 a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+      a[i] = *reinterpret_cast<const float4 *>(&in[4 * ts + i][k]);
+      b[i] = *reinterpret_cast<const float4 *>(&w[tn + 16 * i][k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+      {
+        acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+        acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+        acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+        acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+      }
   }
-  red[threadIdx.x] = acc;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      float h, dh;
+      silu_pair(acc[i][j], h, dh);
+      out[4 * ts + i][tn + 16 * j] = round_out ? bf16_round(h) : h;
+      der[4 * ts + i][tn + 16 * j] = dh;
+    }
+}
+
+// der = (dz W) * der: the gradient of the layer below's pre-activations; thread (ts, tk)
+// does samples 4 ts .. 4 ts + 3 and inputs 4 tk .. 4 tk + 3
+__device__ __forceinline__ void
+tile_backward(const float (*dz)[TLD], const float (*w)[TLD], float (*der)[TLD])
+{
+  const int ts = threadIdx.x >> 4, k0 = 4 * (threadIdx.x & 15);
+  float acc[4][4] = {};
+#pragma unroll 4
+  for (int n = 0; n < SG_H; n += 4)
+  {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+      a[i] = *reinterpret_cast<const float4 *>(&dz[4 * ts + i][n]);
+      b[i] = *reinterpret_cast<const float4 *>(&w[n + i][k0]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+      const float an[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+      {
+        acc[i][0] = fmaf(an[q], b[q].x, acc[i][0]);
+        acc[i][1] = fmaf(an[q], b[q].y, acc[i][1]);
+        acc[i][2] = fmaf(an[q], b[q].z, acc[i][2]);
+        acc[i][3] = fmaf(an[q], b[q].w, acc[i][3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+  {
+    float4 * o = reinterpret_cast<float4 *>(&der[4 * ts + i][k0]);
+    const float4 s = *o;
+    *o = make_float4(acc[i][0] * s.x, acc[i][1] * s.y, acc[i][2] * s.z, acc[i][3] * s.w);
+  }
+}
+
+// g += dz^T h over the tile: outputs 4 (t / 16) .. + 3, inputs 4 (t % 16) .. + 3
+__device__ __forceinline__ void
+tile_weights(const float (*dz)[TLD], const float (*h)[TLD], float (&g)[4][4])
+{
+  const int n0 = 4 * (threadIdx.x >> 4), k0 = 4 * (threadIdx.x & 15);
+#pragma unroll 8
+  for (int s = 0; s < TS; ++s)
+  {
+    const float4 a = *reinterpret_cast<const float4 *>(&dz[s][n0]);
+    const float4 b = *reinterpret_cast<const float4 *>(&h[s][k0]);
+    const float an[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+      g[i][0] = fmaf(an[i], b.x, g[i][0]);
+      g[i][1] = fmaf(an[i], b.y, g[i][1]);
+      g[i][2] = fmaf(an[i], b.z, g[i][2]);
+      g[i][3] = fmaf(an[i], b.w, g[i][3]);
+    }
+  }
+}
+
+// Forward and backward pass of the batch rows (*step * B + i) % n of a training set
+// (step NULL: row i), block b on tiles b, b + gridDim.x, ...: the block's gradients
+// into P[b][SG_NPARAM], its loss into lossp[b].  `wts`: the samples' weights of output 0
+// (NULL: 1); output 1 is weighted by w1.  quant: the hidden layers' weights and inputs
+// are rounded to BF16.
+__global__ void __launch_bounds__(256, 1)
+train_pass_kernel(const float * xs, const float * ys, const float * wts, long long n, long long B, const int * step,
+                  const float * params, int quant, float w1, float * P, float * lossp)
+{
+  extern __shared__ __align__(16) unsigned char train_smem[];
+  TrainSmem & m = *reinterpret_cast<TrainSmem *>(train_smem);
+  const int t = threadIdx.x;
+  for (int i = t; i < SG_H * SG_H; i += 256)
+  {
+    const float a = params[OFF.w2 + i], b = params[OFF.w3 + i];
+    m.w2[i >> 6][i & 63] = quant ? bf16_round(a) : a;
+    m.w3[i >> 6][i & 63] = quant ? bf16_round(b) : b;
+  }
+  if (t < 128)
+  {
+    m.w1[t] = params[OFF.w1 + t];
+    m.w4[t] = params[OFF.w4 + t];
+  }
+  if (t < 64)
+  {
+    m.b1[t] = params[OFF.b1 + t];
+    m.b2[t] = params[OFF.b2 + t];
+    m.b3[t] = params[OFF.b3 + t];
+  }
+  if (t < 2)
+    m.b4[t] = params[OFF.b4 + t];
+
+  float g2[4][4] = {}, g3[4][4] = {};
+  float gb1 = 0.0f, gb2 = 0.0f, gb3 = 0.0f; // output t % 64, a quarter of the tile's samples
+  float g1 = 0.0f, g4 = 0.0f, gb4 = 0.0f;   // threads below 128 (gb4: 2)
+  float loss = 0.0f;
+  const long long first = step ? (long long)*step * B : 0;
+  for (long long at = (long long)blockIdx.x * TS; at < B; at += (long long)gridDim.x * TS)
+  {
+    __syncthreads(); // the weights are in place; the last tile is done
+    const int rows = int(B - at < TS ? B - at : TS);
+    if (t < TS)
+    {
+      // rows past the batch's end hold zeros and get zero gradients
+      const long long src = t < rows ? (first + at + t) % n : 0;
+      m.x[t][0] = t < rows ? xs[2 * src] : 0.0f;
+      m.x[t][1] = t < rows ? xs[2 * src + 1] : 0.0f;
+      m.y[t][0] = t < rows ? ys[2 * src] : 0.0f;
+      m.y[t][1] = t < rows ? ys[2 * src + 1] : 0.0f;
+      m.wt[t] = t < rows && wts ? wts[src] : 1.0f;
+    }
+    __syncthreads();
+    for (int i = t; i < TS * SG_H; i += 256)
+    {
+      const int s = i >> 6, j = i & 63;
+      const float z = fmaf(m.x[s][1], m.w1[2 * j + 1], fmaf(m.x[s][0], m.w1[2 * j], m.b1[j]));
+      float h, dh;
+      silu_pair(z, h, dh);
+      m.h[0][s][j] = quant ? bf16_round(h) : h;
+      m.d[0][s][j] = dh;
+    }
+    __syncthreads();
+    tile_forward(m.h[0], m.w2, m.b2, m.h[1], m.d[1], quant != 0);
+    __syncthreads();
+    tile_forward(m.h[1], m.w3, m.b3, m.h[2], m.d[2], false);
+    __syncthreads();
+    if (t < 2 * TS)
+    {
+      // output layer, loss and its gradient 2 w (o - y) / B
+      const int s = t >> 1, c = t & 1;
+      float o = m.b4[c];
+#pragma unroll 4
+      for (int k = 0; k < SG_H; k += 4)
+      {
+        const float4 a = *reinterpret_cast<const float4 *>(&m.h[2][s][k]);
+        const float4 b = *reinterpret_cast<const float4 *>(&m.w4[c * SG_H + k]);
+        o = fmaf(a.x, b.x, o);
+        o = fmaf(a.y, b.y, o);
+        o = fmaf(a.z, b.z, o);
+        o = fmaf(a.w, b.w, o);
+      }
+      const float wc = c ? w1 : m.wt[s];
+      const float e = s < rows ? o - m.y[s][c] : 0.0f;
+      m.dO[s][c] = 2.0f * wc * e / float(B);
+      loss += wc * e * e;
+    }
+    __syncthreads();
+    if (t < 2 * SG_H)
+    {
+      const int c = t >> 6, k = t & 63;
+      for (int s = 0; s < TS; ++s)
+        g4 = fmaf(m.dO[s][c], m.h[2][s][k], g4);
+    }
+    else if (t < 2 * SG_H + 2)
+      for (int s = 0; s < TS; ++s)
+        gb4 += m.dO[s][t - 2 * SG_H];
+    for (int i = t; i < TS * SG_H; i += 256)
+    {
+      const int s = i >> 6, k = i & 63;
+      const float g = fmaf(m.dO[s][1], m.w4[SG_H + k], m.dO[s][0] * m.w4[k]);
+      m.d[2][s][k] = g * m.d[2][s][k];
+    }
+    __syncthreads();
+    tile_weights(m.d[2], m.h[1], g3);
+    tile_backward(m.d[2], m.w3, m.d[1]);
+    __syncthreads();
+    tile_weights(m.d[1], m.h[0], g2);
+    tile_backward(m.d[1], m.w2, m.d[0]);
+    __syncthreads();
+    if (t < 2 * SG_H)
+      for (int s = 0; s < TS; ++s)
+        g1 = fmaf(m.d[0][s][t >> 1], m.x[s][t & 1], g1);
+    for (int s = 16 * (t >> 6); s < 16 * (t >> 6) + 16; ++s)
+    {
+      gb1 += m.d[0][s][t & 63];
+      gb2 += m.d[1][s][t & 63];
+      gb3 += m.d[2][s][t & 63];
+    }
+  }
+  float * out = P + (long long)blockIdx.x * SG_NPARAM;
+  const int n0 = 4 * (t >> 4), k0 = 4 * (t & 15);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      out[OFF.w2 + (n0 + i) * SG_H + k0 + j] = g2[i][j];
+      out[OFF.w3 + (n0 + i) * SG_H + k0 + j] = g3[i][j];
+    }
+  if (t < 2 * SG_H)
+  {
+    out[OFF.w1 + t] = g1;
+    out[OFF.w4 + t] = g4;
+  }
+  else if (t < 2 * SG_H + 2)
+    out[OFF.b4 + t - 2 * SG_H] = gb4;
+  const float gb[3] = {gb1, gb2, gb3};
+  const int off[3] = {OFF.b1, OFF.b2, OFF.b3};
+  for (int l = 0; l < 3; ++l)
+  {
+    __syncthreads();
+    m.red[t >> 6][t & 63] = gb[l];
+    __syncthreads();
+    if (t < SG_H)
+      out[off[l] + t] = ((m.red[0][t] + m.red[1][t]) + m.red[2][t]) + m.red[3][t];
+  }
+  __syncthreads();
+  float * red = &m.red[0][0];
+  red[t] = loss;
   __syncthreads();
   for (int w = 128; w > 0; w >>= 1)
   {
-    if (threadIdx.x < w)
-      red[threadIdx.x] += red[threadIdx.x + w];
+    if (t < w)
+      red[t] += red[t + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0)
-    loss_partial[blockIdx.x] = red[0];
+  if (t == 0)
+    lossp[blockIdx.x] = red[0];
 }
 
-// dX[s][k] = sum_n dZ[s][n] W[n][k], then times silu'(Zprev[s][k])
-__global__ void
-dense_bwd_data(const float * dZ, const float * W, int N, int K, long long B, const float * Zprev, float * dX,
-               int quant)
+// the blocks' gradients added in block order
+__device__ __forceinline__ float
+sum_blocks(const float * P, int parts, int i)
 {
-  extern __shared__ float sw[];
-  for (int i = threadIdx.x; i < N * K; i += blockDim.x)
-    sw[i] = quant ? bf16_round(W[i]) : W[i];
-  __syncthreads();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= B * K)
-    return;
-  const long long s = idx / K;
-  const int k = int(idx % K);
   float g = 0.0f;
-  const float * dz = dZ + s * N;
-  for (int n = 0; n < N; ++n)
-    g = fmaf(dz[n], sw[n * K + k], g);
-  dX[idx] = g * silu_d(Zprev[idx]);
-}
-
-// partial weight gradients over a slice of the batch: P[p][n][k] = sum_s dZ[s][n] X[s][k]
-// and P[p][N][n] for the bias; grid (N, parts)
-__global__ void
-dense_bwd_weight(const float * dZ, const float * X, int N, int K, long long B, int parts, float * P, int quant)
-{
-  const int n = blockIdx.x;
-  const int p = blockIdx.y;
-  const long long s0 = B * p / parts, s1 = B * (p + 1) / parts;
-  const int k = threadIdx.x; // blockDim.x == 64 >= K
-  float acc = 0.0f, accb = 0.0f;
-  for (long long s = s0; s < s1; ++s)
-  {
-    const float d = dZ[s * N + n];
-    if (k < K)
-      acc = fmaf(d, quant ? bf16_round(X[s * K + k]) : X[s * K + k], acc);
-    accb += d;
-  }
-  const long long base = (long long)p * (N * K + N);
-  if (k < K)
-    P[base + n * K + k] = acc;
-  if (k == 0)
-    P[base + N * K + n] = accb;
-}
-
-// G[i] = sum_p P[p][i] in order; scatter into the flat gradient vector
-__global__ void
-reduce_parts(const float * P, int count, int parts, float * gW, float * gb, int N, int K)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count)
-    return;
-  float a = 0.0f;
+#pragma unroll 8
   for (int p = 0; p < parts; ++p)
-    a += P[(long long)p * count + i];
-  if (i < N * K)
-    gW[i] = a;
-  else
-    gb[i - N * K] = a;
+    g += P[(long long)p * SG_NPARAM + i];
+  return g;
 }
 
 __global__ void
-adam_step(float * w, const float * g, float * m, float * v, int n, const int * step, float lr, float b1, float b2,
-          float eps_adam, float lr_final_frac, int total_steps)
+gradient_sum_kernel(const float * P, int parts, float * g)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
+  if (i < SG_NPARAM)
+    g[i] = sum_blocks(P, parts, i);
+}
+
+// gradient sum and Adam step; the last block to finish counts the step
+__global__ void
+adam_step(float * w, const float * P, int parts, float * m, float * v, int * step, unsigned int * done, float lr,
+          float b1, float b2, float eps_adam, float lr_final_frac, int total_steps)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int t = *step + 1;
-  // cosine decay from lr to lr * lr_final_frac
-  const float prog = fminf(1.0f, float(t) / float(total_steps));
-  const float lrt = lr * (lr_final_frac + (1.0f - lr_final_frac) * 0.5f * (1.0f + cosf(3.14159265f * prog)));
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float mh = mi / (1.0f - powf(b1, float(t)));
-  const float vh = vi / (1.0f - powf(b2, float(t)));
-  w[i] -= lrt * mh / (sqrtf(vh) + eps_adam);
-}
-
-__global__ void
-bump_step(int * step)
-{
-  *step += 1;
-}
-
-// gather batch rows by a device-side step counter (epoch-cyclic)
-__global__ void
-gather_batch(const float * x, const float * y, const float * w, long long n, long long B, const int * step, float * bx,
-             float * by, float * bw)
-{
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B)
-    return;
-  const long long src = ((long long)(*step) * B + i) % n;
-  bx[2 * i] = x[2 * src];
-  bx[2 * i + 1] = x[2 * src + 1];
-  by[2 * i] = y[2 * src];
-  by[2 * i + 1] = y[2 * src + 1];
-  if (w)
-    bw[i] = w[src];
+  if (i < SG_NPARAM)
+  {
+    // cosine decay from lr to lr * lr_final_frac
+    const float prog = fminf(1.0f, float(t) / float(total_steps));
+    const float lrt = lr * (lr_final_frac + (1.0f - lr_final_frac) * 0.5f * (1.0f + cosf(3.14159265f * prog)));
+    const float gi = sum_blocks(P, parts, i);
+    const float mi = b1 * m[i] + (1.0f - b1) * gi;
+    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    const float mh = mi / (1.0f - powf(b1, float(t)));
+    const float vh = vi / (1.0f - powf(b2, float(t)));
+    w[i] -= lrt * mh / (sqrtf(vh) + eps_adam);
+  }
+  __syncthreads(); // the block has read the step
+  if (threadIdx.x == 0 && atomicAdd(done, 1u) == gridDim.x - 1)
+  {
+    *done = 0u;
+    *step = t;
+  }
 }
 
 // flat parameters -> inference layout
@@ -451,112 +636,77 @@ surrogate_net_bytes()
   return sizeof(SurrogateNet);
 }
 
-// One forward + backward pass over a batch (device buffers), gradients into g.
-struct TrainBuffers
-{
-  long long B;
-  int parts;
-  float *bx, *by;                // batch inputs/targets [B][2]
-  float * bw;                    // per-sample loss weights of output 0 [B], or NULL
-  float *z1, *h1, *z2, *h2, *z3, *h3, *o;
-  float *d3, *d2, *d1, *dO;      // gradients of pre-activations
-  float * P;                     // partial weight gradients
-  float * lossp;                 // loss partials
-};
-
+// blocks of a training pass over B samples: one per SM of the current device at most
 static cudaError_t
-fwd_bwd(const float * w, float * g, const TrainBuffers & t, int quant, float w_tau, cudaStream_t st)
+train_blocks(long long B, int & blocks)
 {
-  const long long B = t.B;
-  const int T = 256;
-  auto blocks = [&](long long n) { return (unsigned int)((n + T - 1) / T); };
-  dense_fwd<<<blocks(B * 64), T, 64 * 2 * 4, st>>>(t.bx, 2, w + OFF.w1, w + OFF.b1, 64, B, t.z1, t.h1, 1, 0);
-  dense_fwd<<<blocks(B * 64), T, 64 * 64 * 4, st>>>(t.h1, 64, w + OFF.w2, w + OFF.b2, 64, B, t.z2, t.h2, 1, quant);
-  dense_fwd<<<blocks(B * 64), T, 64 * 64 * 4, st>>>(t.h2, 64, w + OFF.w3, w + OFF.b3, 64, B, t.z3, t.h3, 1, quant);
-  dense_fwd<<<blocks(B * 2), T, 2 * 64 * 4, st>>>(t.h3, 64, w + OFF.w4, w + OFF.b4, 2, B, t.o, nullptr, 0, 0);
-  loss_grad<<<64, 256, 0, st>>>(t.o, t.by, t.bw, B, w_tau, t.dO, t.lossp);
-  // output layer
-  dense_bwd_weight<<<dim3(2, t.parts), 64, 0, st>>>(t.dO, t.h3, 2, 64, B, t.parts, t.P, 0);
-  reduce_parts<<<(2 * 64 + 2 + 127) / 128, 128, 0, st>>>(t.P, 2 * 64 + 2, t.parts, g + OFF.w4, g + OFF.b4, 2, 64);
-  dense_bwd_data<<<blocks(B * 64), T, 2 * 64 * 4, st>>>(t.dO, w + OFF.w4, 2, 64, B, t.z3, t.d3, 0);
-  // hidden layer 3
-  dense_bwd_weight<<<dim3(64, t.parts), 64, 0, st>>>(t.d3, t.h2, 64, 64, B, t.parts, t.P, quant);
-  reduce_parts<<<(64 * 64 + 64 + 127) / 128, 128, 0, st>>>(t.P, 64 * 64 + 64, t.parts, g + OFF.w3, g + OFF.b3, 64, 64);
-  dense_bwd_data<<<blocks(B * 64), T, 64 * 64 * 4, st>>>(t.d3, w + OFF.w3, 64, 64, B, t.z2, t.d2, quant);
-  // hidden layer 2
-  dense_bwd_weight<<<dim3(64, t.parts), 64, 0, st>>>(t.d2, t.h1, 64, 64, B, t.parts, t.P, quant);
-  reduce_parts<<<(64 * 64 + 64 + 127) / 128, 128, 0, st>>>(t.P, 64 * 64 + 64, t.parts, g + OFF.w2, g + OFF.b2, 64, 64);
-  dense_bwd_data<<<blocks(B * 64), T, 64 * 64 * 4, st>>>(t.d2, w + OFF.w2, 64, 64, B, t.z1, t.d1, quant);
-  // input layer
-  dense_bwd_weight<<<dim3(64, t.parts), 64, 0, st>>>(t.d1, t.bx, 64, 2, B, t.parts, t.P, 0);
-  reduce_parts<<<(64 * 2 + 64 + 127) / 128, 128, 0, st>>>(t.P, 64 * 2 + 64, t.parts, g + OFF.w1, g + OFF.b1, 64, 2);
-  return cudaGetLastError();
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  e = e ? e : cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  e = e ? e
+        : cudaFuncSetAttribute(train_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TrainSmem)));
+  blocks = int(std::min<long long>((B + TS - 1) / TS, std::max(sms, 1)));
+  return e;
 }
 
-// ---- exported to the C ABI layer (mtg_api.cu)
-
-struct SurrogateTrainer
+// device memory cut from one allocation, freed with it
+struct Arena
 {
-  float * w = nullptr; // parameters
-  void * net = nullptr;
-  bool trained = false;
+  unsigned char * base = nullptr;
+  size_t size = 0;
+  ~Arena()
+  {
+    if (base)
+      cudaFree(base);
+  }
+  // bytes of an array, kept 256-byte aligned
+  size_t add(size_t bytes)
+  {
+    const size_t at = size;
+    size += (bytes + 255) / 256 * 256;
+    return at;
+  }
+  cudaError_t alloc() { return cudaMalloc(&base, size); }
+  float * at(size_t o) { return reinterpret_cast<float *>(base + o); }
 };
+
+constexpr unsigned int PARAM_BLOCKS = (SG_NPARAM + 127) / 128;
+
+// ---- exported to the C ABI layer (mtg_api.cu)
 
 cudaError_t
 surrogate_gradients(const float * params_h, const float * x_h, const float * y_h, long long n, float w_tau,
                     float * loss_h, float * grads_h)
 {
-  TrainBuffers t{};
-  t.B = n;
-  t.parts = 4;
-  std::vector<void *> allocs;
-  auto alloc = [&](float *& p, size_t count) {
-    cudaError_t e = cudaMalloc(&p, count * sizeof(float));
-    allocs.push_back(p);
+  int blocks = 0;
+  cudaError_t e = train_blocks(n, blocks);
+  if (e)
     return e;
-  };
-  float *w = nullptr, *g = nullptr;
-  cudaError_t e = cudaSuccess;
   const size_t B = size_t(n);
-  e = e ? e : alloc(w, SG_NPARAM);
-  e = e ? e : alloc(g, SG_NPARAM);
-  e = e ? e : alloc(t.bx, 2 * B);
-  e = e ? e : alloc(t.by, 2 * B);
-  e = e ? e : alloc(t.z1, 64 * B);
-  e = e ? e : alloc(t.h1, 64 * B);
-  e = e ? e : alloc(t.z2, 64 * B);
-  e = e ? e : alloc(t.h2, 64 * B);
-  e = e ? e : alloc(t.z3, 64 * B);
-  e = e ? e : alloc(t.h3, 64 * B);
-  e = e ? e : alloc(t.o, 2 * B);
-  e = e ? e : alloc(t.d3, 64 * B);
-  e = e ? e : alloc(t.d2, 64 * B);
-  e = e ? e : alloc(t.d1, 64 * B);
-  e = e ? e : alloc(t.dO, 2 * B);
-  e = e ? e : alloc(t.P, size_t(t.parts) * (64 * 64 + 64));
-  e = e ? e : alloc(t.lossp, 64);
-  if (!e)
-    e = cudaMemcpy(w, params_h, SG_NPARAM * 4, cudaMemcpyHostToDevice);
-  if (!e)
-    e = cudaMemcpy(t.bx, x_h, 2 * B * 4, cudaMemcpyHostToDevice);
-  if (!e)
-    e = cudaMemcpy(t.by, y_h, 2 * B * 4, cudaMemcpyHostToDevice);
-  if (!e)
-    e = fwd_bwd(w, g, t, 0, w_tau, nullptr);
-  if (!e)
-    e = cudaMemcpy(grads_h, g, SG_NPARAM * 4, cudaMemcpyDeviceToHost);
+  Arena a;
+  const size_t ow = a.add(4 * SG_NPARAM), og = a.add(4 * SG_NPARAM), ox = a.add(8 * B), oy = a.add(8 * B),
+               oP = a.add(4 * size_t(SG_NPARAM) * blocks), ol = a.add(4 * size_t(blocks));
+  if ((e = a.alloc()) != cudaSuccess)
+    return e;
+  e = cudaMemcpy(a.at(ow), params_h, SG_NPARAM * 4, cudaMemcpyHostToDevice);
+  e = e ? e : cudaMemcpy(a.at(ox), x_h, 8 * B, cudaMemcpyHostToDevice);
+  e = e ? e : cudaMemcpy(a.at(oy), y_h, 8 * B, cudaMemcpyHostToDevice);
+  if (e)
+    return e;
+  train_pass_kernel<<<blocks, 256, sizeof(TrainSmem)>>>(a.at(ox), a.at(oy), nullptr, n, n, nullptr, a.at(ow), 0, w_tau,
+                                                        a.at(oP), a.at(ol));
+  gradient_sum_kernel<<<PARAM_BLOCKS, 128>>>(a.at(oP), blocks, a.at(og));
+  e = cudaGetLastError();
+  e = e ? e : cudaMemcpy(grads_h, a.at(og), SG_NPARAM * 4, cudaMemcpyDeviceToHost);
+  std::vector<float> lp(static_cast<size_t>(blocks));
+  e = e ? e : cudaMemcpy(lp.data(), a.at(ol), 4 * lp.size(), cudaMemcpyDeviceToHost);
   if (!e)
   {
-    float lp[64];
-    e = cudaMemcpy(lp, t.lossp, sizeof lp, cudaMemcpyDeviceToHost);
     double s = 0.0;
     for (float v : lp)
       s += v;
     *loss_h = float(s / double(n));
   }
-  for (void * p : allocs)
-    if (p)
-      cudaFree(p);
   return e;
 }
 
@@ -567,136 +717,85 @@ surrogate_train(long long n_train, int batch, int epochs, int qat_epochs, float 
                 double * train_seconds)
 {
   upload_nodes_once();
+  int blocks = 0;
+  cudaError_t e = train_blocks(batch, blocks);
+  if (e)
+    return e;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0);
-  std::vector<void *> allocs;
-  auto alloc = [&](void ** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    allocs.push_back(*p);
-    return e;
-  };
-  cudaError_t e = cudaSuccess;
-  float *x = nullptr, *y = nullptr, *wts = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
-  int * step = nullptr;
-  TrainBuffers t{};
-  t.B = batch;
-  t.parts = 32;
-  const size_t B = size_t(batch);
-  e = e ? e : alloc((void **)&x, 2 * sizeof(float) * n_train);
-  e = e ? e : alloc((void **)&y, 2 * sizeof(float) * n_train);
-  if (weighting)
-  {
-    e = e ? e : alloc((void **)&wts, sizeof(float) * n_train);
-    e = e ? e : alloc((void **)&t.bw, 4 * B);
-  }
-  e = e ? e : alloc((void **)&g, 4 * SG_NPARAM);
-  e = e ? e : alloc((void **)&m, 4 * SG_NPARAM);
-  e = e ? e : alloc((void **)&v, 4 * SG_NPARAM);
-  e = e ? e : alloc((void **)&step, 4);
-  float ** bufs[] = {&t.bx, &t.by, &t.o, &t.dO};
-  for (float ** p : bufs)
-    e = e ? e : alloc((void **)p, 2 * 4 * B);
-  float ** wide[] = {&t.z1, &t.h1, &t.z2, &t.h2, &t.z3, &t.h3, &t.d3, &t.d2, &t.d1};
-  for (float ** p : wide)
-    e = e ? e : alloc((void **)p, 64 * 4 * B);
-  e = e ? e : alloc((void **)&t.P, 4 * size_t(t.parts) * (64 * 64 + 64));
-  e = e ? e : alloc((void **)&t.lossp, 4 * 64);
-  if (e)
-  {
-    for (void * p : allocs)
-      if (p)
-        cudaFree(p);
-    return e;
-  }
-  uint32_t k0 = uint32_t(seed), k1 = uint32_t(seed >> 32) ^ 0x53474E4Eu;
-  make_training_data<<<(unsigned int)((n_train + 127) / 128), 128>>>(n_train, k0, k1, 0u, target, x, y, wts);
-  if (wts)
-  {
-    // normalise the weights to mean 1 over the training set
-    std::vector<float> hw(n_train);
-    e = cudaMemcpy(hw.data(), wts, sizeof(float) * n_train, cudaMemcpyDeviceToHost);
-    double sum = 0.0;
-    for (float w : hw)
-      sum += double(w);
-    if (!e && sum > 0.0)
-      scale_weights<<<(unsigned int)((n_train + 255) / 256), 256>>>(wts, n_train, float(double(n_train) / sum));
-  }
-  // initial weights: uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) from a host LCG
+  const size_t n = size_t(n_train);
+  Arena a;
+  const size_t ox = a.add(8 * n), oy = a.add(8 * n), owt = a.add(weighting ? 4 * n : 0), om = a.add(4 * SG_NPARAM),
+               ov = a.add(4 * SG_NPARAM), ostep = a.add(8), oP = a.add(4 * size_t(SG_NPARAM) * blocks),
+               ol = a.add(4 * size_t(blocks));
+  e = a.alloc();
   std::vector<float> w0(SG_NPARAM, 0.0f);
-  uint64_t st = seed * 6364136223846793005ull + 1442695040888963407ull;
-  auto uni = [&]() {
-    st = st * 6364136223846793005ull + 1442695040888963407ull;
-    return float((st >> 11) * (1.0 / 9007199254740992.0)) * 2.0f - 1.0f;
-  };
-  for (int i = 0; i < 128; ++i)
-    w0[OFF.w1 + i] = uni() * 1.2f;
-  for (int i = 0; i < 4096; ++i)
-    w0[OFF.w2 + i] = uni() * 0.3f;
-  for (int i = 0; i < 4096; ++i)
-    w0[OFF.w3 + i] = uni() * 0.3f;
-  for (int i = 0; i < 128; ++i)
-    w0[OFF.w4 + i] = uni() * 0.2f;
-  cudaMemcpy(params_dev, w0.data(), 4 * SG_NPARAM, cudaMemcpyHostToDevice);
-  cudaMemset(m, 0, 4 * SG_NPARAM);
-  cudaMemset(v, 0, 4 * SG_NPARAM);
-  cudaMemset(step, 0, 4);
   const long long steps_per_epoch = std::max<long long>(1, n_train / batch);
   const int total = int(steps_per_epoch * epochs);
-  cudaStream_t s;
-  cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-  cudaGraphExec_t exec[2] = {nullptr, nullptr};
-  for (int q = 0; q < 2 && !e; ++q)
-  {
-    cudaGraph_t graph;
-    e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-    if (e)
-      break;
-    gather_batch<<<(unsigned int)((batch + 255) / 256), 256, 0, s>>>(x, y, wts, n_train, batch, step, t.bx, t.by,
-                                                                      t.bw);
-    fwd_bwd(params_dev, g, t, q, w_tau, s);
-    adam_step<<<(SG_NPARAM + 255) / 256, 256, 0, s>>>(params_dev, g, m, v, SG_NPARAM, step, lr, 0.9f, 0.999f, 1e-8f,
-                                                      0.02f, total);
-    bump_step<<<1, 1, 0, s>>>(step);
-    e = cudaStreamEndCapture(s, &graph);
-    if (!e)
-      e = cudaGraphInstantiate(&exec[q], graph, 0);
-    cudaGraphDestroy(graph);
-  }
-  for (int it = 0; it < total && !e; ++it)
-  {
-    const bool quant = it >= int(steps_per_epoch * (epochs - qat_epochs));
-    e = cudaGraphLaunch(exec[quant ? 1 : 0], s);
-  }
-  if (!e)
-    e = cudaStreamSynchronize(s);
   if (!e)
   {
-    float lp[64];
-    cudaMemcpy(lp, t.lossp, sizeof lp, cudaMemcpyDeviceToHost);
+    float *x = a.at(ox), *y = a.at(oy), *wts = weighting ? a.at(owt) : nullptr, *m = a.at(om), *v = a.at(ov);
+    int * step = reinterpret_cast<int *>(a.at(ostep)); // and the finished blocks of a step
+    const uint32_t k0 = uint32_t(seed), k1 = uint32_t(seed >> 32) ^ 0x53474E4Eu;
+    make_training_data<<<(unsigned int)((n_train + 127) / 128), 128>>>(n_train, k0, k1, 0u, target, x, y, wts);
+    // initial weights: uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) from a host LCG
+    uint64_t st = seed * 6364136223846793005ull + 1442695040888963407ull;
+    auto uni = [&]() {
+      st = st * 6364136223846793005ull + 1442695040888963407ull;
+      return float((st >> 11) * (1.0 / 9007199254740992.0)) * 2.0f - 1.0f;
+    };
+    for (int i = 0; i < 128; ++i)
+      w0[OFF.w1 + i] = uni() * 1.2f;
+    for (int i = 0; i < 4096; ++i)
+      w0[OFF.w2 + i] = uni() * 0.3f;
+    for (int i = 0; i < 4096; ++i)
+      w0[OFF.w3 + i] = uni() * 0.3f;
+    for (int i = 0; i < 128; ++i)
+      w0[OFF.w4 + i] = uni() * 0.2f;
+    if (wts)
+    {
+      // normalise the weights to mean 1 over the training set
+      std::vector<float> hw(n);
+      e = cudaMemcpy(hw.data(), wts, 4 * n, cudaMemcpyDeviceToHost);
+      double sum = 0.0;
+      for (float w : hw)
+        sum += double(w);
+      if (!e && sum > 0.0)
+        scale_weights<<<(unsigned int)((n_train + 255) / 256), 256>>>(wts, n_train, float(double(n_train) / sum));
+    }
+    e = e ? e : cudaMemcpy(params_dev, w0.data(), 4 * SG_NPARAM, cudaMemcpyHostToDevice);
+    e = e ? e : cudaMemset(a.base + om, 0, oP - om); // Adam's moments and the step count
+    for (int it = 0; it < total && !e; ++it)
+    {
+      const int quant = it >= int(steps_per_epoch * (epochs - qat_epochs));
+      train_pass_kernel<<<blocks, 256, sizeof(TrainSmem)>>>(x, y, wts, n_train, batch, step, params_dev, quant, w_tau,
+                                                            a.at(oP), a.at(ol));
+      adam_step<<<PARAM_BLOCKS, 128>>>(params_dev, a.at(oP), blocks, m, v, step,
+                                       reinterpret_cast<unsigned int *>(step) + 1, lr, 0.9f, 0.999f, 1e-8f, 0.02f,
+                                       total);
+      e = cudaGetLastError();
+    }
+  }
+  if (!e)
+  {
+    std::vector<float> lp(static_cast<size_t>(blocks));
+    e = cudaMemcpy(lp.data(), a.at(ol), 4 * lp.size(), cudaMemcpyDeviceToHost);
     double sum = 0.0;
     for (float val : lp)
       sum += val;
     *final_loss = sum / double(batch);
-    e = launch_pack_net(params_dev, net_dev, nullptr);
   }
-  if (!e)
-    e = cudaDeviceSynchronize();
+  e = e ? e : launch_pack_net(params_dev, net_dev, nullptr);
+  e = e ? e : cudaDeviceSynchronize();
   cudaEventRecord(e1);
   cudaEventSynchronize(e1);
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, e0, e1);
   *train_seconds = ms / 1e3;
-  for (auto & ge : exec)
-    if (ge)
-      cudaGraphExecDestroy(ge);
-  cudaStreamDestroy(s);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  for (void * p : allocs)
-    if (p)
-      cudaFree(p);
   return e;
 }
 
