@@ -41,26 +41,89 @@ struct P64
   int tag;       // IonBase::_tag: cluster index where a followed recoil was created, else -1
 };
 
-// proton electronic stopping in one element (material.C:134-158)
+// proton electronic stopping in one element (material.C:134-158) at pe >= 25 keV/u
+// before the velocity factor, lpe = log(pe)
+MTG_HD double
+proton_stop64_above(const StopPair & sp, double pe, double lpe)
+{
+  const double sl = sp.pcoef[0] * exp64(sp.pcoef[1] * lpe) + sp.pcoef[2] * exp64(sp.pcoef[3] * lpe);
+  const double sh = sp.pcoef[4] / exp64(sp.pcoef[5] * lpe) * log64(sp.pcoef[6] / pe + sp.pcoef[7] * pe);
+  return sl * sh / (sl + sh);
+}
+
+// proton electronic stopping in one element: up to 25 keV/u the value there (sp.s25)
+// times a power of the energy
 MTG_HD double
 proton_stop64(const StopPair & sp, double e)
 {
-  const double pe = e > 25.0 ? e : 25.0;
-  const double lpe = log64(pe);
-  const double sl = sp.pcoef[0] * exp64(sp.pcoef[1] * lpe) + sp.pcoef[2] * exp64(sp.pcoef[3] * lpe);
-  const double sh = sp.pcoef[4] / exp64(sp.pcoef[5] * lpe) * log64(sp.pcoef[6] / pe + sp.pcoef[7] * pe);
-  double s = sl * sh / (sl + sh);
   if (e <= 25.0)
-    s *= pow64(e / 25.0, sp.velpwr);
-  return s;
+    return sp.s25 * pow64(e / 25.0, sp.velpwr);
+  return proton_stop64_above(sp, e, log64(e));
 }
 
-// electronic stopping of species sc with energy E [eV] in element sp, in the
-// reference's units (material.C:161-281, result * 10)
+// relative velocity of a heavy ion over its Z1^(2/3), before the cut at yrcut
 MTG_HD double
-ion_stop64(const SpeciesConst & sc, const StopPair & sp, double E)
+reduced_velocity64(const SpeciesConst & sc, const StopPair & sp, double e)
 {
-  const double e = E * sc.inv_m1k; // keV/u
+  const double vf = sp.vfermi;
+  const double v = sqrt(e / 25.0) / vf;
+  const double v2 = v * v;
+  double vr;
+  if (v >= 1.0)
+    vr = v * vf * (1.0 + 1.0 / (5.0 * v2));
+  else
+    vr = (3.0 * vf / 4.0) * (1.0 + (2.0 * v2 / 3.0) - v2 * v2 / 15.0);
+  return vr / sc.cb2;
+}
+
+// effective charge fraction of a heavy ion at the (cut) reduced velocity yr, before its
+// Z1^2 correction
+MTG_HD double
+zeta64(const SpeciesConst & sc, const StopPair & sp, double yr)
+{
+  const double vf = sp.vfermi;
+  const double yr03 = pow64(yr, 0.3);
+  double a = -0.803 * yr03 + 1.3167 * yr03 * yr03 + 0.38157 * yr + 0.008983 * yr * yr;
+  double q = 1.0 - exp64(-(a < 50.0 ? a : 50.0));
+  q = q < 0.0 ? 0.0 : (q > 1.0 ? 1.0 : q);
+  const double b = sc.bq;
+  const double l0 = (0.8 - q * sc.l0a) / sc.cb;
+  double l1;
+  if (q < 0.2)
+    l1 = 0.0;
+  else if (q < sc.qlo)
+    l1 = b * (q - 0.2) / sc.qden;
+  else if (q < sc.qhi)
+    l1 = b;
+  else
+    l1 = b * (1.0 - q) / sc.qden2;
+  const double l0f = l0 * sc.lfctr;
+  const double l = l1 > l0f ? l1 : l0f;
+  const double w = 4.0 * l * vf / 1.919;
+  return q + sp.inv2vf2 * (1.0 - q) * log64(1.0 + w * w);
+}
+
+// zeta Z1 with the Z1^2 correction, le = log(e)
+MTG_HD double
+corrected_charge64(const SpeciesConst & sc, const StopPair & sp, double zeta, double le)
+{
+  const double t = 7.6 - (le > 0.0 ? le : 0.0);
+  zeta *= 1.0 + sc.inv_z1sq * sp.zc * exp64(-(t * t));
+  return zeta * sc.fz1;
+}
+
+// electronic stopping of species sc with e = E inv_m1k [keV/u] (le = log(e), heavy ions)
+// in element sp, in the reference's units (material.C:161-281, result * 10).
+//
+// GB300 runs FP64 at 2 lanes per SM and clock, and nearly every collision of a cascade
+// is of a slow heavy particle, for which most of the formula does not depend on the
+// energy: those parts are taken from StopPair, where the host has put the same
+// expressions' values (bit for bit: prepare_stop_pair64).  With the rejection passes and
+// the Newton loop's test off the FP64 unit: 2000 Ag 200 keV into Si 188 -> 153 ms, a
+// stopping curve of 10^6 energies 1.31 -> 0.68 ms with its copies.
+MTG_HD double
+ion_stop64(const SpeciesConst & sc, const StopPair & sp, double e, double le)
+{
   double se;
   if (sc.branch == STOP_H)
     se = proton_stop64(sp, e);
@@ -79,58 +142,78 @@ ion_stop64(const SpeciesConst & sc, const StopPair & sp, double E)
     if (e <= 1.0)
       se *= sqrt(e);
   }
+  else if (e < sp.e_clamp)
+  {
+    double low = sp.low_cut;
+    if (le > 0.0)
+    {
+      const double zf = corrected_charge64(sc, sp, sp.zeta_cut, le);
+      low = sp.sp_eee * (zf * zf);
+    }
+    se = low * exp64(sp.power * (le - sp.ln_eee));
+  }
   else
   {
-    const double vf = sp.vfermi;
-    const double v = sqrt(e / 25.0) / vf;
-    const double v2 = v * v;
-    double vr;
-    if (v >= 1.0)
-      vr = v * vf * (1.0 + 1.0 / (5.0 * v2));
-    else
-      vr = (3.0 * vf / 4.0) * (1.0 + (2.0 * v2 / 3.0) - v2 * v2 / 15.0);
-    double yr = vr / sc.cb2;
+    double yr = reduced_velocity64(sc, sp, e);
     if (yr < sp.yrcut)
       yr = sp.yrcut;
-    const double yr03 = pow64(yr, 0.3);
-    double a = -0.803 * yr03 + 1.3167 * yr03 * yr03 + 0.38157 * yr + 0.008983 * yr * yr;
-    double q = 1.0 - exp64(-(a < 50.0 ? a : 50.0));
-    q = q < 0.0 ? 0.0 : (q > 1.0 ? 1.0 : q);
-    const double b = sc.bq;
-    const double l0 = (0.8 - q * sc.l0a) / sc.cb;
-    double l1;
-    if (q < 0.2)
-      l1 = 0.0;
-    else if (q < sc.qlo)
-      l1 = b * (q - 0.2) / sc.qden;
-    else if (q < sc.qhi)
-      l1 = b;
-    else
-      l1 = b * (1.0 - q) / sc.qden2;
-    const double l0f = l0 * sc.lfctr;
-    const double l = l1 > l0f ? l1 : l0f;
-    const double w = 4.0 * l * vf / 1.919;
-    double zeta = q + sp.inv2vf2 * (1.0 - q) * log64(1.0 + w * w);
-    const double le = log64(e);
-    const double t = 7.6 - (le > 0.0 ? le : 0.0);
-    zeta *= 1.0 + sc.inv_z1sq * sp.zc * exp64(-(t * t));
-    const double zf = zeta * sc.fz1;
+    const double zf = corrected_charge64(sc, sp, zeta64(sc, sp, yr), le);
     if (yr <= sp.yrcut)
-      se = sp.sp_eee * (zf * zf) * exp64(sp.power * (le - log64(sp.eee)));
+      se = sp.sp_eee * (zf * zf) * exp64(sp.power * (le - sp.ln_eee));
     else
       se = proton_stop64(sp, e) * (zf * zf);
   }
   return se * 10.0;
 }
 
+// the energy-independent values of ion_stop64 (host)
+inline void
+prepare_stop_pair64(const SpeciesConst & sc, StopPair & sp)
+{
+  sp.s25 = proton_stop64_above(sp, 25.0, log64(25.0));
+  sp.ln_eee = log64(sp.eee);
+  sp.zeta_cut = zeta64(sc, sp, sp.yrcut);
+  const double zf = corrected_charge64(sc, sp, sp.zeta_cut, 0.0);
+  sp.low_cut = sp.sp_eee * (zf * zf);
+  // The reduced velocity rises with the energy (its derivative is positive on both
+  // branches, which meet at v = 1) and is computed to a few 1e-16: where it is below
+  // yrcut (1 - 1e-12) it is below yrcut as computed at every smaller energy, too.  Just
+  // below the energy where it reaches yrcut, from the branches' inverses:
+  const double X = sp.yrcut * sc.cb2 / sp.vfermi; // relative velocity over the Fermi velocity
+  double s = 0.0;                                 // v^2
+  if (X >= 1.2)
+  {
+    const double v = 0.5 * (X + sqrt(X * X - 0.8));
+    s = v * v;
+  }
+  else if (X > 0.75)
+    s = 5.0 - sqrt(25.0 - 15.0 * (4.0 * X / 3.0 - 1.0));
+  const double e = 25.0 * s * sp.vfermi * sp.vfermi * (1.0 - 1e-6);
+  sp.e_clamp = reduced_velocity64(sc, sp, e) < sp.yrcut * (1.0 - 1e-12) ? e : 0.0;
+}
+
 // MaterialBase::getrstop (material.C:114-121), eV/Angstrom
 MTG_HD double
 material_stop64(const SpeciesConst & sc, const MatConst & mc, double E)
 {
+  const double e = E * sc.inv_m1k; // keV/u
+  const double le = sc.branch == STOP_HEAVY ? log64(e) : 0.0;
   double se = 0.0;
   for (int j = 0; j < mc.nel; ++j)
-    se += ion_stop64(sc, mc.sp[j], E) * mc.el[j].t;
+    se += ion_stop64(sc, mc.sp[j], e, le) * mc.el[j].t;
   return se * mc.arho;
+}
+
+// a / b > c for a, b >= 0 and c > 0, as the rounded quotient says it.  Integer compares of
+// a with b c settle all but a few in 10^6 cases without the division.
+MTG_HD bool
+exceeds_ratio64(double a, double b, double c)
+{
+  const uint64_t x = double_to_bits(a), y = double_to_bits(b * c);
+  const uint64_t inf = 0x7ff0000000000000ull;
+  if (x - y + 0x100000000ull > 0x200000000ull && x < inf && y < inf) // apart by 2^-21 or more
+    return x > y;
+  return a / b > c;
 }
 
 // Scattering (trim.C:172-271) for the universal (pot 0), Moliere (1) or C-Kr (2)
@@ -197,7 +280,7 @@ scatter64(double eps, double b, double & s2, double & ct, double & st, int & nit
     q = fr / fr1;
     r -= q;
     ++niter;
-  } while (fabs(q / r) > 0.001 && niter < 100);
+  } while (exceeds_ratio64(fabs(q), fabs(r), 0.001) && niter < 100);
   const double roc = -2.0 * (eps - v) / v1;
   const double sqe = sqrt(eps);
   double cc, aa, ff;
@@ -225,6 +308,21 @@ scatter64(double eps, double b, double & s2, double & ct, double & st, int & nit
   s2 = 1.0 - c2;
   ct = 2.0 * c2 - 1.0;
   st = sqrt(1.0 - ct * ct);
+}
+
+// coordinate 2 u - 1 of a point in the cube, u = (x + 1) / 2^32, times 2^31: an exact
+// integer, read off the double whose low word is x
+MTG_HD double
+ball_coordinate64(uint32_t x)
+{
+  return bits_to_double(0x4330000000000000ull | x) - (0x1p52 + 2147483647.0);
+}
+
+// the coordinate itself, to 2^-24
+MTG_HD float
+ball_coordinate32(uint32_t x)
+{
+  return float(int32_t(x ^ 0x80000000u)) * 0x1p-31f;
 }
 
 // One collision.  `mats` points at this species' MatConst row of the simulation
@@ -278,14 +376,17 @@ collide64(P64 & p, uint32_t ic, double r1, const SimDesc & sim, const SpeciesCon
   // impact parameter and target atom (trim.C:143-160)
   const U4 d0 = draw_block(p.key, ic, 0u, k0, k1);
   const double r2 = u53(d0.x, d0.y);
-  double hh = u53(d0.z, d0.w);
   const double pimp = pmax * sqrt(r2);
   int nn = 0;
-  for (; nn < mc.nel - 1; ++nn)
+  if (mc.nel > 1)
   {
-    hh -= mc.el[nn].t;
-    if (hh <= 0)
-      break;
+    double hh = u53(d0.z, d0.w);
+    for (; nn < mc.nel - 1; ++nn)
+    {
+      hh -= mc.el[nn].t;
+      if (hh <= 0)
+        break;
+    }
   }
   const ElemConst & el = mc.el[nn];
   eps = el.fi * p.E;
@@ -327,20 +428,31 @@ collide64(P64 & p, uint32_t ic, double r1, const SimDesc & sim, const SpeciesCon
   rec.species = el.rspecies;
   rec.tag = -1; // a new IonBase (ion.C:26)
 
-  // random unit vector perpendicular to dir by unit-ball rejection (trim.C:322-333)
+  // random unit vector perpendicular to dir by unit-ball rejection (trim.C:322-333).
+  // The ball's points are kept 2^31 times too large (exact, and the unit vector's bits do
+  // not depend on it), and single precision tells all but one in 10^5 of the points
+  // inside the ball from those outside: a warp passes five times or so until its last
+  // lane is inside, 21 FP64 operations each time.
   double px, py, pz, nrm;
   uint32_t pass = 0;
   do
   {
-    double rx, ry, rz;
+    U4 dr;
+    bool outside;
     do
     {
-      const U4 dr = draw_block(p.key, ic, 1u + pass, k0, k1);
+      dr = draw_block(p.key, ic, 1u + pass, k0, k1);
       ++pass;
-      rx = 2.0 * u32d(dr.x) - 1.0;
-      ry = 2.0 * u32d(dr.y) - 1.0;
-      rz = 2.0 * u32d(dr.z) - 1.0;
-    } while (rx * rx + ry * ry + rz * rz > 1.0 && pass < 64);
+      const float fx = ball_coordinate32(dr.x), fy = ball_coordinate32(dr.y), fz = ball_coordinate32(dr.z);
+      const float f2 = fx * fx + fy * fy + fz * fz; // to 1e-6
+      outside = f2 > 1.0f;
+      if (f2 > 0.99999f && f2 < 1.00001f)
+      {
+        const double rx = ball_coordinate64(dr.x), ry = ball_coordinate64(dr.y), rz = ball_coordinate64(dr.z);
+        outside = rx * rx + ry * ry + rz * rz > 0x1p62;
+      }
+    } while (outside && pass < 64);
+    const double rx = ball_coordinate64(dr.x), ry = ball_coordinate64(dr.y), rz = ball_coordinate64(dr.z);
     px = p.dy * rz - p.dz * ry;
     py = p.dz * rx - p.dx * rz;
     pz = p.dx * ry - p.dy * rx;

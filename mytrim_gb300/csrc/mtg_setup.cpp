@@ -1,6 +1,8 @@
 // Host-side table construction for the cascade engine (see mtg_setup.h).
 #include "mtg_setup.h"
 
+#include "mtg_collide64.cuh"
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -120,6 +122,7 @@ make_stop_pair(const mtg_scoef_row * rows, const SpeciesConst & sc, int Z2)
   p.zc = 0.18 + 0.0015 * double(Z2);
   p.hez = 0.007 + 0.00005 * double(Z2);
   p.Z2 = Z2;
+  prepare_stop_pair64(sc, p);
   return p;
 }
 

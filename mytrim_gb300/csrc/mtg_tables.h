@@ -54,6 +54,13 @@ struct StopPair
   double power;     // low-velocity exponent (material.C:264-267)
   double zc;        // 0.18 + 0.0015 Z2
   double hez;       // 0.007 + 0.00005 Z2 (helium)
+  // values that the stopping of slow ions repeats, each the result of the expressions it
+  // stands for (mtg_collide64.cuh): below e_clamp [keV/u] the reduced velocity of a heavy
+  // ion is surely cut to yrcut, its charge state a constant (zeta_cut, before the Z1^2
+  // correction) and below 1 keV/u the whole factor of the power law (low_cut)
+  double e_clamp, zeta_cut, low_cut;
+  double ln_eee;    // log(eee)
+  double s25;       // proton stopping at 25 keV/u before the velocity factor
   int Z2;
   int pad;
 };

@@ -240,6 +240,60 @@ main(int argc, char ** argv)
     printf("%lld %lld\n", checked, bad);
     return bad ? 1 : 0;
   }
+  if (argc >= 4 && std::string(argv[2]) == "--stopcheck")
+  {
+    // the stopping with its precomputed parts against the same expressions evaluated at
+    // every energy, around each of its limits, and the ratio test against the division;
+    // prints how many were compared and how many differ
+    const int n = atoi(argv[3]);
+    unsigned long long st = 1;
+    auto uniform = [&]() {
+      st = st * 6364136223846793005ull + 1442695040888963407ull;
+      return double(st >> 11) * (1.0 / 9007199254740992.0);
+    };
+    long long checked = 0, bad = 0;
+    for (int Z1 = 1; Z1 <= MTG_SCOEF_ROWS; ++Z1)
+      for (int Z2 = 1; Z2 <= MTG_SCOEF_ROWS; ++Z2)
+      {
+        const SpeciesConst sc = make_species(rows, Z1, rows[Z1 - 1].m1);
+        const StopPair sp = make_stop_pair(rows, sc, Z2);
+        const double limits[3] = {sp.e_clamp, 25.0, 1.0};
+        for (int i = 0; i < n; ++i)
+        {
+          double e = std::pow(10.0, -5.0 + 11.0 * uniform());
+          if (i % 2 && limits[i / 2 % 3] > 0.0)
+            e = limits[i / 2 % 3] * (1.0 + (uniform() - 0.5) * (i % 4 == 1 ? 1e-5 : 1e-14));
+          const double le = log64(e);
+          double want;
+          if (sc.branch == STOP_HEAVY)
+          {
+            double yr = reduced_velocity64(sc, sp, e);
+            yr = yr < sp.yrcut ? sp.yrcut : yr;
+            const double zf = corrected_charge64(sc, sp, zeta64(sc, sp, yr), le);
+            double proton = proton_stop64_above(sp, e > 25.0 ? e : 25.0, log64(e > 25.0 ? e : 25.0));
+            if (e <= 25.0)
+              proton *= pow64(e / 25.0, sp.velpwr);
+            want = (yr <= sp.yrcut ? sp.sp_eee * (zf * zf) * exp64(sp.power * (le - log64(sp.eee)))
+                                   : proton * (zf * zf)) *
+                   10.0;
+          }
+          else
+          {
+            StopPair whole = sp; // H and He: only the proton stopping at 25 keV/u is precomputed
+            whole.s25 = proton_stop64_above(sp, 25.0, log64(25.0));
+            want = ion_stop64(sc, whole, e, le);
+          }
+          ++checked;
+          bad += double_to_bits(ion_stop64(sc, sp, e, le)) != double_to_bits(want);
+          const double r = std::exp(10.0 * uniform() - 5.0);
+          const double q = 0.001 * r * (i % 2 ? 1.0 + (uniform() - 0.5) * 4e-16 * (1 << i % 30) : uniform() * 2.0);
+          ++checked;
+          bad += exceeds_ratio64(q, r, 0.001) != (q / r > 0.001);
+        }
+      }
+    printf("%lld %lld\n", checked, bad);
+    return bad ? 1 : 0;
+  }
   if (argc >= 3 && std::string(argv[2]) == "--scatter")
   {
     // lines "eps b" -> s2; an optional argument after --scatter picks the potential
