@@ -14,6 +14,12 @@
 namespace mtg
 {
 
+__device__ __forceinline__ float
+record_energy(const P64 & p)
+{
+  return float(p.E);
+}
+
 struct Fp64Policy
 {
   using Particle = P64;
