@@ -106,13 +106,14 @@ struct Recoil32
   int tag;
 };
 
-// E -= d, keeping the rounding remainder (TwoSum followed by FastTwoSum)
+// E -= d for |d| <= E, keeping the rounding remainder: FastTwoSum twice (Dekker 1971;
+// with the larger term first it gives TwoSum's remainder in half its operations, 2.7 %
+// of the kernel's time on Ag into Si)
 __device__ __forceinline__ void
 ff_sub(float & hi, float & lo, float d)
 {
   const float s = hi - d;
-  const float bb = s - hi;
-  const float err = (hi - (s - bb)) + (-d - bb);
+  const float err = (hi - s) - d;
   const float l = lo + err;
   const float h = s + l;
   lo = l - (h - s);
@@ -254,24 +255,24 @@ phase_b32(P32 & p, const PhaseA32 & a, const Sim32 & sim, const Tables32 & t, co
 
   // energy transfer, electronic loss, momenta (trim.C:275-296)
   float den = a.ec * s2 * E;
-  if (dee >= E)
   {
-    dee = E + p.El;
-    p.E = 0.0f;
-    p.El = 0.0f;
+    float h = p.E, l = p.El;
+    ff_sub(h, l, dee);
+    const bool all = dee >= E;
+    dee = all ? E + p.El : dee;
+    p.E = all ? 0.0f : h;
+    p.El = all ? 0.0f : l;
   }
-  else
-    ff_sub(p.E, p.El, dee);
   sink.eel(dee, p.x, p.y, p.z);
   const float p1 = sqrtf(a.two_m1 * p.E);
-  if (den >= p.E)
   {
-    den = p.E + p.El;
-    p.E = 0.0f;
-    p.El = 0.0f;
+    float h = p.E, l = p.El;
+    ff_sub(h, l, den);
+    const bool all = den >= p.E;
+    den = all ? p.E + p.El : den;
+    p.E = all ? 0.0f : h;
+    p.El = all ? 0.0f : l;
   }
-  else
-    ff_sub(p.E, p.El, den);
   const float p2 = sqrtf(a.two_m1 * p.E);
 
   // recoil at the pre-flight position (trim.C:306-318)
@@ -317,13 +318,12 @@ phase_b32(P32 & p, const PhaseA32 & a, const Sim32 & sim, const Tables32 & t, co
   // CUT boundaries (trim.C:344-352)
   if (sim.any_cut)
   {
-    const float pos[3] = {p.x, p.y, p.z};
-    for (int i = 0; i < 3; ++i)
-      if (sim.bc[i] == 2 && (pos[i] > sim.w[i] || pos[i] < 0.0f))
-      {
-        sink.lost(p.E + p.El + den, p, mc.Z1, mc.m1);
-        return CF_DONE;
-      }
+    if (p.x > sim.cut_hi[0] || p.x < sim.cut_lo[0] || p.y > sim.cut_hi[1] || p.y < sim.cut_lo[1] ||
+        p.z > sim.cut_hi[2] || p.z < sim.cut_lo[2])
+    {
+      sink.lost(p.E + p.El + den, p, mc.Z1, mc.m1);
+      return CF_DONE;
+    }
   }
 
   // fate of recoil and projectile (trim.C:357-411)
@@ -385,15 +385,15 @@ phase_b32(P32 & p, const PhaseA32 & a, const Sim32 & sim, const Tables32 & t, co
 }
 
 // resident 128-thread blocks per SM the register budget of each feature level is cut
-// for: lean, mid and events 8 (64 registers), full and clusters+events 7 (72), geometry
-// and clusters 6 (80); the surrogate's tensor-core fragments need 128 registers
+// for: lean, mid and events 8 (64 registers; 7 measured 1.4 % slower on Ag into Si, 9
+// 0.2 % faster there and 10 % slower on the 4096-simulation batch), the others 7 (72; 6
+// measured 4.5 % slower on Xe into UO2 with bubbles); the surrogate's tensor-core
+// fragments need 128 registers (5 blocks 18 % slower, 3 blocks 8 %)
 template <int LVL, bool SURROGATE>
 struct Blocks32
 {
-  static constexpr int value = SURROGATE ? 4
-                               : LVL == LVL_LEAN || LVL == LVL_MID || LVL == LVL_EVENTS ? 8
-                               : LVL == LVL_GEO || LVL == LVL_CLU                       ? 6
-                                                                                        : 7;
+  static constexpr int value =
+      SURROGATE ? 4 : LVL == LVL_LEAN || LVL == LVL_MID || LVL == LVL_EVENTS ? 8 : 7;
 };
 
 template <int LVL, bool SURROGATE, bool ONE>

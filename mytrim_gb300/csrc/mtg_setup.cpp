@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstring>
 #include <fstream>
+#include <limits>
 #include <sstream>
 #include <string>
 #include <unordered_map>
@@ -276,6 +277,8 @@ build_fp32_tables(const HostTables & t, std::vector<Mat32> & mats, std::vector<M
       o.w[k] = float(d.w[k]);
       o.bc[k] = d.bc[k];
       o.any_cut |= d.bc[k] == 2;
+      o.cut_lo[k] = d.bc[k] == 2 ? 0.0f : -std::numeric_limits<float>::infinity();
+      o.cut_hi[k] = d.bc[k] == 2 ? o.w[k] : std::numeric_limits<float>::infinity();
     }
     o.n_layers = d.n_layers;
     o.n_mat = d.n_mat;

@@ -249,6 +249,7 @@ struct Sim32
   int n_layers, n_mat, mat_base, species_base;
   float Ef, flscale, tau, cw; // flscale = 1 / length scale
   int range_mode, primaries_only, any_cut, geometry;
+  float cut_lo[3], cut_hi[3]; // where a CUT boundary takes members out; infinities on other axes
   int follow_gen, kp_gen, potential, pad1;
   // sampleClusters geometry (see SimDesc)
   int kn[3];
