@@ -83,7 +83,7 @@ struct mtg_ctx
   bool prepared = false;
   bool launched = false;
   // device buffers
-  DevBuf d_sims, d_prim_end, d_species, d_mats, d_row_species, d_stop;
+  DevBuf d_sims, d_order, d_order_end, d_species, d_mats, d_row_species, d_stop;
   DevBuf d_mats32, d_cold32, d_sims32;
   DevBuf d_sg_params, d_sg_net; // surrogate network
   DevBuf d_vox, d_vox_range, d_vox_sum, d_vox_part; // energy-deposition voxels
@@ -273,7 +273,8 @@ fill_params(mtg_ctx * ctx, EngineParams & prm)
   std::memset(&prm, 0, sizeof prm);
   prm.sims = ptr<SimDesc>(ctx->d_sims);
   prm.n_sims = int(t.sims.size());
-  prm.sim_prim_end = ptr<long long>(ctx->d_prim_end);
+  prm.order = ptr<int>(ctx->d_order);
+  prm.order_end = ptr<long long>(ctx->d_order_end);
   if (ctx->cfg.precision == MTG_PREC_FP64)
   {
     prm.species = ptr<SpeciesConst>(ctx->d_species);
@@ -502,7 +503,7 @@ mtg_destroy(mtg_ctx * ctx)
   if (!ctx)
     return MTG_OK;
   cudaSetDevice(ctx->device);
-  DevBuf * bufs[] = {&ctx->d_sims,   &ctx->d_prim_end, &ctx->d_species, &ctx->d_mats,    &ctx->d_row_species,
+  DevBuf * bufs[] = {&ctx->d_sims,   &ctx->d_order, &ctx->d_order_end, &ctx->d_species, &ctx->d_mats,    &ctx->d_row_species,
                      &ctx->d_stop,   &ctx->p_vac,      &ctx->p_coll,    &ctx->p_eel,     &ctx->p_enuc,
                      &ctx->p_fx,     &ctx->p_fy,       &ctx->p_fz,      &ctx->p_state,   &ctx->d_totals,
                      &ctx->d_hist,   &ctx->d_err,      &ctx->d_counters, &ctx->d_stacks, &ctx->d_ovf0,
@@ -595,7 +596,8 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
   const size_t ns = t.sims.size();
   const size_t np = size_t(std::max<long long>(t.total_primaries, 1));
   CK(ensure(ctx->d_sims, sizeof(SimDesc) * ns));
-  CK(ensure(ctx->d_prim_end, sizeof(long long) * ns));
+  CK(ensure(ctx->d_order, sizeof(int) * ns));
+  CK(ensure(ctx->d_order_end, sizeof(long long) * ns));
   CK(ensure(ctx->d_species, sizeof(SpeciesConst) * t.species.size()));
   CK(ensure(ctx->d_mats, sizeof(MatConst) * t.mats.size()));
   CK(ensure(ctx->p_vac, 8 * np));
@@ -645,7 +647,8 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
                            ptr<uint32_t>(ctx->d_cl_mask));
   }
   CK(h2d(ctx, ctx->d_sims.p, ctx->sims_dev.data(), sizeof(SimDesc) * ns));
-  CK(h2d(ctx, ctx->d_prim_end.p, t.prim_end.data(), sizeof(long long) * ns));
+  CK(h2d(ctx, ctx->d_order.p, t.order.data(), sizeof(int) * ns));
+  CK(h2d(ctx, ctx->d_order_end.p, t.order_end.data(), sizeof(long long) * ns));
   CK(h2d(ctx, ctx->d_species.p, t.species.data(), sizeof(SpeciesConst) * t.species.size()));
   CK(h2d(ctx, ctx->d_mats.p, t.mats.data(), sizeof(MatConst) * t.mats.size()));
 
@@ -940,7 +943,7 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
       hist[i] = (long long)h[i];
   }
   size_t bytes = 0;
-  DevBuf * bufs[] = {&ctx->d_sims,   &ctx->d_prim_end, &ctx->d_species, &ctx->d_mats,    &ctx->d_row_species,
+  DevBuf * bufs[] = {&ctx->d_sims,   &ctx->d_order, &ctx->d_order_end, &ctx->d_species, &ctx->d_mats,    &ctx->d_row_species,
                      &ctx->d_stop,   &ctx->p_vac,      &ctx->p_coll,    &ctx->p_eel,     &ctx->p_enuc,
                      &ctx->p_fx,     &ctx->p_fy,       &ctx->p_fz,      &ctx->p_state,   &ctx->d_totals,
                      &ctx->d_hist,   &ctx->d_err,      &ctx->d_counters, &ctx->d_stacks, &ctx->d_ovf0,

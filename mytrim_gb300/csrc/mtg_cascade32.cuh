@@ -550,9 +550,10 @@ cascade32_kernel(const __grid_constant__ EngineParams prm, const __grid_constant
           }
           else
           {
-            const long long g = base + r;
-            const int s = !ONE && prm.n_sims > 1 ? find_sim(prm.sim_prim_end, prm.n_sims, g) : 0;
+            long long g = base + r, first = 0;
+            const int s = !ONE && prm.n_sims > 1 ? find_sim(prm, g, first) : 0;
             const SimDesc & d = ONE ? one.desc : prm.sims[s];
+            g += d.prim_begin - first;
             p.x = float(d.pos[0]);
             p.y = float(d.pos[1]);
             p.z = float(d.pos[2]);

@@ -55,7 +55,10 @@ struct EngineParams
 {
   const SimDesc * sims;
   int n_sims;
-  const long long * sim_prim_end; // exclusive prefix end of each simulation's primaries
+  // the order in which the simulations' primaries are started: simulation order[i] has
+  // the work indexes from order_end[i - 1] to order_end[i]
+  const int * order;
+  const long long * order_end;
   const SpeciesConst * species;
   const MatConst * mats;
   int stage_tables;               // stage species+mats of simulation 0 into shared memory
@@ -300,9 +303,12 @@ lanemask_lt()
   return m;
 }
 
+// the simulation of work index g; `first`: its first work index
 __device__ __forceinline__ int
-find_sim(const long long * ends, int n, long long g)
+find_sim(const EngineParams & prm, long long g, long long & first)
 {
+  const long long * ends = prm.order_end;
+  const int n = prm.n_sims;
   int lo = 0, hi = n - 1;
   while (lo < hi)
   {
@@ -312,7 +318,8 @@ find_sim(const long long * ends, int n, long long g)
     else
       lo = mid + 1;
   }
-  return lo;
+  first = lo > 0 ? ends[lo - 1] : 0;
+  return prm.order[lo];
 }
 
 // Plain FP64 accumulator (FP64 engine)
@@ -1149,8 +1156,9 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
             start_member(in_records[g]);
           else
           {
-            const int s = prm.n_sims > 1 ? find_sim(prm.sim_prim_end, prm.n_sims, g) : 0;
-            start_member(Pol::make_primary(prm.sims[s], s, g));
+            long long first = 0;
+            const int s = prm.n_sims > 1 ? find_sim(prm, g, first) : 0;
+            start_member(Pol::make_primary(prm.sims[s], s, prm.sims[s].prim_begin + (g - first)));
           }
           live = true;
         }

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <fstream>
 #include <limits>
+#include <numeric>
 #include <sstream>
 #include <string>
 #include <unordered_map>
@@ -508,7 +509,7 @@ build_tables(const mtg_scoef_row * rows, const mtg_config & cfg, const mtg_sim *
 {
   // clear, keeping the vectors' storage for the next batch
   out.sims.clear();
-  out.prim_end.clear();
+  out.order_end.clear();
   out.species.clear();
   out.mats.clear();
   out.stop_row_mat.clear();
@@ -554,7 +555,7 @@ build_tables(const mtg_scoef_row * rows, const mtg_config & cfg, const mtg_sim *
     out.species.reserve(nsp);
     out.mats.reserve(nmat);
     out.sims.reserve(size_t(n_sims));
-    out.prim_end.reserve(size_t(n_sims));
+    out.order_end.reserve(size_t(n_sims));
   }
   // (species, material) -> index of its first MatConst: equal pairs across the
   // simulations of a batch share the derived constants and the stopping-table row
@@ -871,7 +872,6 @@ build_tables(const mtg_scoef_row * rows, const mtg_config & cfg, const mtg_sim *
       out.any_evac = 1;
     out.members_est += double(s.n_primaries) * expected_members(s);
     prim += s.n_primaries;
-    out.prim_end.push_back(prim);
     out.sims.push_back(d);
     out.emax = std::max(out.emax, s.ion.E);
   }
@@ -887,6 +887,15 @@ build_tables(const mtg_scoef_row * rows, const mtg_config & cfg, const mtg_sim *
     return MTG_ERR_BAD_INPUT;
   }
   out.total_primaries = prim;
+  // long cascades start first: at the end of a batch the warps finish on short ones
+  // (4096 simulations of 1 keV to 1 MeV, 590,000 primaries: 249 -> 212 ms)
+  out.order.resize(size_t(n_sims));
+  std::iota(out.order.begin(), out.order.end(), 0);
+  std::stable_sort(out.order.begin(), out.order.end(),
+                   [&](int a, int b) { return out.sims[size_t(a)].E0 > out.sims[size_t(b)].E0; });
+  long long end = 0;
+  for (int s : out.order)
+    out.order_end.push_back(end += out.sims[size_t(s)].n_primaries);
   out.members_est = prim > 0 ? out.members_est / double(prim) : 1.0;
   out.hist_total = hist;
   return MTG_OK;

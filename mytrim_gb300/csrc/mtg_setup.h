@@ -15,7 +15,8 @@ namespace mtg
 struct HostTables
 {
   std::vector<SimDesc> sims;
-  std::vector<long long> prim_end;        // exclusive end of each simulation's primaries
+  std::vector<int> order;                 // the simulations by falling ion energy, and
+  std::vector<long long> order_end;       // the exclusive ends of their primaries in that order
   std::vector<SpeciesConst> species;
   std::vector<MatConst> mats;
   long long total_primaries = 0;

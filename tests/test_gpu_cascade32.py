@@ -62,3 +62,22 @@ def test_events_alone_equal_among_others(engine_lib, name):
     for f in logs[0].dtype.names:
         if f != "pad":
             assert np.array_equal(logs[0][f], logs[1][f]), f
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_batch_started_by_energy_equals_each_alone(engine_lib, precision):
+    """A batch starts its simulations by falling energy; every simulation's primaries keep
+    their own streams and tally slots, also beside one without primaries."""
+    sims = [W.boron_implant(7), _arsenic(n_primaries=0), W.cu_self_ion(3, E=20e3), _arsenic(n_primaries=5),
+            W.cu_self_ion(2, E=80e3), _arsenic(n_primaries=1)]
+    e = Engine(precision=precision, seed=12)
+    batch = e.run(sims)
+    per = e.primaries(0, sum(s.n_primaries for s in sims))
+    at = 0
+    for i, s in enumerate(sims):
+        lead = [_arsenic(n_primaries=0)] * i  # the streams are keyed by the simulation's number
+        alone = e.run(lead + [s])[i]
+        assert _whole(batch[i]) == _whole(alone), i
+        assert per["vacancies"][at:at + s.n_primaries].sum() == alone["vacancies"]
+        at += s.n_primaries
+    e.close()
