@@ -131,14 +131,19 @@ struct EngineParams
 // the move (share_min): a mailbox per warp, because a common list of chunks that all idle
 // warps watched was slower by a factor of a hundred than no sharing at all.
 //
+// The notes are single releasing stores: a fence (__threadfence) also empties the SM's L1,
+// from which all its warps read their tables, and is left to the receipt of a letter.
+//
 // Nothing here depends on another warp's progress but the last step of a letter, between
 // a sender's claim of a mailbox and its note that the recoils are in it.  An idle warp
 // leaves when all others are idle or gone, or after PATIENCE ns; it gives up its mailbox
 // first, by a compare-and-swap that fails if a sender has claimed it.
 //
 // FP64 kernel, Ag 200 keV into Si: 64 primaries 55 -> 42 ms, 1000 107 -> 87 ms, 2000
-// 153 -> 139 ms.  The FP32 kernel goes without: a warp's iteration takes it 2 us instead of
-// 30 and more, a letter 7, and the loop lost 2 to 4 % to the code's mere presence.
+// 153 -> 139 ms.  With the network, 50,000 Ag 113 -> 100 ms.  The exact FP32 kernel goes
+// without: a warp's iteration takes it 2 us instead of 30 and more, a letter 7; 10^4 Au
+// 1 MeV with voxels gained 8 % and Xe into bubbles 6, 10^4 Cu 100 keV lost 14 %, 10^6 B 7
+// and the 4096-simulation batch 12.
 struct PoolControl
 {
   unsigned int hungry, gone; // warps waiting, warps that left
@@ -154,6 +159,7 @@ struct PoolControl
 template <class Rec>
 struct RecoilPool
 {
+  static constexpr int NO_SHARING = 0x7fffffff; // EngineParams::share_after
   static constexpr unsigned int PATIENCE = 20000000u;
   static constexpr unsigned int WAITING = 1u, CLAIMED = 2u, LEFT = 3u, FULL = 0x100u; // mailbox states; FULL + records
   static constexpr int RING_BITS = 14; // more entries than the GPU holds warps
@@ -170,6 +176,8 @@ struct RecoilPool
   // number, 0: none will come
   static __device__ __forceinline__ int wait(const EngineParams & prm, unsigned int warp, Rec * stack, int lane)
   {
+    if (prm.share_after == NO_SHARING)
+      return 0;
     unsigned int k = 0;
     if (lane == 0)
     {
@@ -178,13 +186,13 @@ struct RecoilPool
       unsigned int * box = prm.pool_box + warp;
       const volatile unsigned int * vbox = box;
       *reinterpret_cast<volatile unsigned int *>(box) = WAITING;
-      __threadfence();
       atomicAdd(&ctl->hungry, 1u);
       const unsigned int t = atomicAdd(&ctl->tail, 1u);
-      *reinterpret_cast<volatile unsigned long long *>(prm.pool_ring + (t & (RING - 1))) =
-          (unsigned long long)tag(prm, t) << 32 | (warp + 1u);
-      __threadfence();
-      atomicAdd(&ctl->avail, 1);
+      asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(prm.pool_ring + (t & (RING - 1))),
+                   "l"((unsigned long long)tag(prm, t) << 32 | (warp + 1u))
+                   : "memory");
+      int before;
+      asm volatile("atom.add.release.gpu.global.s32 %0, [%1], 1;" : "=r"(before) : "l"(&ctl->avail) : "memory");
       unsigned int slept = 0;
       bool claimed = false;
       for (int i = 0; i < (1 << 20); ++i)
@@ -218,7 +226,8 @@ struct RecoilPool
         atomicAdd(&ctl->gone, 1u);
       }
       atomicSub(&ctl->hungry, 1u);
-      __threadfence();
+      if (k != 0u)
+        __threadfence(); // the letter's recoils after its note
     }
     k = __shfl_sync(0xffffffffu, k, 0);
     __syncwarp();
@@ -281,10 +290,10 @@ struct RecoilPool
       return top;
     if (lane < k)
       reinterpret_cast<Rec *>(prm.pool_recs)[to * 32 + lane] = stack[lane];
-    __threadfence();
     __syncwarp();
     if (lane == 0)
-      *reinterpret_cast<volatile unsigned int *>(prm.pool_box + to) = FULL + (unsigned int)k;
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(prm.pool_box + to), "r"(FULL + (unsigned int)k)
+                   : "memory");
     if (lane < m)
       stack[lane] = stack[top - m + lane];
     __syncwarp();
