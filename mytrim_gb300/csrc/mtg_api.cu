@@ -13,6 +13,7 @@
 #include "mytrim_gpu.h"
 #include "mtg_engine.cuh"
 #include "mtg_kernels.h"
+#include "mtg_reduce.cuh"
 #include "mtg_setup.h"
 
 using namespace mtg;
@@ -659,13 +660,13 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
   CK(h2d(ctx, ctx->d_species.p, t.species.data(), sizeof(SpeciesConst) * t.species.size()));
   CK(h2d(ctx, ctx->d_mats.p, t.mats.data(), sizeof(MatConst) * t.mats.size()));
 
-  // reduction jobs: contiguous chunks of at most 65536 primaries per simulation
+  // reduction jobs: contiguous chunks of each simulation's primaries
   ctx->jobs.clear();
   ctx->job_first.assign(1, 0);
   for (size_t s = 0; s < ns; ++s)
   {
     const long long b = t.sims[s].prim_begin, n = t.sims[s].n_primaries;
-    const long long chunk = 65536;
+    const long long chunk = reduce_chunk(n);
     for (long long o = 0; o < n; o += chunk)
       ctx->jobs.push_back(ReduceJob{int(s), b + o, b + std::min(n, o + chunk)});
     ctx->job_first.push_back(int(ctx->jobs.size()));

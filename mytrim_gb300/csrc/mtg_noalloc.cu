@@ -11,7 +11,7 @@
 // every GPU that loads the library holds until the process exits.
 //
 // The arithmetic is the one mtg_collect uses (mtg_reduce.cuh, shared with
-// mtg_reduce.cu): chunks of 65536 primaries, each summed by one block in a fixed
+// mtg_reduce.cu): chunks of at most 65536 primaries, each summed by one block in a fixed
 // order, then the chunks in index order with compensated FP64 adds, so the totals
 // are the same bits as the ones mtg_collect reports for a single simulation.
 #include <cuda.h> // CUcontext / CUresult types only: the driver calls are reached through the runtime
@@ -30,7 +30,7 @@ namespace
 {
 
 constexpr int NOALLOC_BLOCK = mtg::RBLOCK;
-constexpr long long NOALLOC_CHUNK = 65536; // primaries per block, as in mtg_collect
+constexpr long long NOALLOC_CHUNK = 65536; // most primaries per block (mtg::reduce_chunk, as in mtg_collect)
 constexpr int NOALLOC_MAX_CHUNKS = 1024;   // at most 67,108,864 primaries per call
 constexpr int NQ = mtg::NQ;
 
@@ -44,10 +44,10 @@ static __device__ __align__(256) double g_noalloc_partials[NOALLOC_MAX_CHUNKS * 
 __global__ void __launch_bounds__(NOALLOC_BLOCK)
 noalloc_chunk_kernel(const unsigned long long * vac, const unsigned long long * coll, const double * eel,
                      const double * enuc, const double * fx, const double * fy, const double * fz,
-                     const int * fstate, long long n, double * partials)
+                     const int * fstate, long long n, long long chunk, double * partials)
 {
-  const long long begin = (long long)blockIdx.x * NOALLOC_CHUNK;
-  const long long end = begin + NOALLOC_CHUNK < n ? begin + NOALLOC_CHUNK : n;
+  const long long begin = (long long)blockIdx.x * chunk;
+  const long long end = begin + chunk < n ? begin + chunk : n;
   mtg::block_sum_primaries(vac, coll, eel, enuc, fx, fy, fz, fstate, begin, end, partials + (long long)blockIdx.x * NQ);
 }
 
@@ -179,10 +179,11 @@ mtg_reduce_primaries_noalloc(const unsigned long long * vacancies, const unsigne
     scratch = c.addr;
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int nchunks = int((n + NOALLOC_CHUNK - 1) / NOALLOC_CHUNK);
+  const long long chunk = mtg::reduce_chunk(n);
+  const int nchunks = int((n + chunk - 1) / chunk);
   if (nchunks > 0)
     noalloc_chunk_kernel<<<nchunks, NOALLOC_BLOCK, 0, st>>>(vacancies, collisions, eel, enuc, x, y, z, state, n,
-                                                            scratch);
+                                                            chunk, scratch);
   noalloc_finish_kernel<<<1, 32, 0, st>>>(scratch, nchunks, out);
   e = cudaGetLastError();
   if (e != cudaSuccess)
