@@ -44,6 +44,39 @@ ensure(DevBuf & b, size_t bytes)
   return e;
 }
 
+// Buffers cut from one allocation, 256-byte aligned, in the order given: small tables that
+// go to the device in one copy, tallies that are cleared by one memset.
+struct Cut
+{
+  DevBuf * b;
+  size_t bytes;
+};
+
+constexpr size_t
+aligned(size_t bytes)
+{
+  return (bytes + 255) / 256 * 256;
+}
+
+cudaError_t
+cut(DevBuf & arena, const std::vector<Cut> & parts)
+{
+  size_t total = 0;
+  for (const Cut & c : parts)
+    total += aligned(c.bytes);
+  const cudaError_t e = ensure(arena, std::max<size_t>(total, 256));
+  if (e != cudaSuccess)
+    return e;
+  char * at = static_cast<char *>(arena.p);
+  for (const Cut & c : parts)
+  {
+    c.b->p = at;
+    c.b->bytes = c.bytes;
+    at += aligned(c.bytes);
+  }
+  return cudaSuccess;
+}
+
 template <class T>
 T *
 ptr(DevBuf & b)
@@ -83,7 +116,12 @@ struct mtg_ctx
   std::vector<Sim32> sm32;
   bool prepared = false;
   bool launched = false;
-  // device buffers
+  // device buffers: d_tables and d_run are allocations, the next two lines and the primaries'
+  // tallies, totals, histograms, error flags, counters and results are cut from them
+  DevBuf d_tables, d_run;
+  std::vector<char> staging; // the tables on their way to d_tables
+  char * h_results = nullptr; // pinned: counters, error flags, totals, sums and voxel sums of a run
+  size_t h_bytes = 0, results_bytes = 0;
   DevBuf d_sims, d_order, d_order_end, d_species, d_mats, d_row_species, d_stop;
   DevBuf d_mats32, d_cold32, d_sims32;
   DevBuf d_sg_params, d_sg_net; // surrogate network
@@ -254,7 +292,6 @@ setup_launch_shape(mtg_ctx * ctx)
   chk(ensure(ctx->d_ovf1, size_t(ctx->ovf_cap) * rec), "overflow allocation");
   if (prec != MTG_PREC_FP32)
   {
-    chk(ensure(ctx->d_pool_ctl, sizeof(PoolControl) * MAX_PASSES), "pool allocation");
     // zeroed once: no entry is valid and no mailbox waits before a warp of a launch says so
     auto zeroed = [&](DevBuf & b, size_t bytes) {
       const size_t before = b.bytes;
@@ -369,7 +406,10 @@ launch_pass(mtg_ctx * ctx, int pass)
   fill_params(ctx, prm);
   unsigned long long * cnt = ptr<unsigned long long>(ctx->d_counters);
   prm.next_primary = cnt + C_NEXT0 + (pass % MAX_PASSES);
-  CK(cudaMemsetAsync(prm.next_primary, 0, sizeof(unsigned long long), ctx->stream));
+  // a run's first two passes find everything cleared
+  const bool again = pass > 1;
+  if (again)
+    CK(cudaMemsetAsync(prm.next_primary, 0, sizeof(unsigned long long), ctx->stream));
   if (ctx->cfg.precision != MTG_PREC_FP32)
   {
     prm.pool = ptr<PoolControl>(ctx->d_pool_ctl) + pass % MAX_PASSES;
@@ -387,12 +427,14 @@ launch_pass(mtg_ctx * ctx, int pass)
     prm.share_after = ctx->cfg.precision == MTG_PREC_FP64 || ctx->tables.emax >= 80e3
                           ? ctx->grid * (ctx->block / 32) / 4
                           : RecoilPool<int>::NO_SHARING;
-    CK(cudaMemsetAsync(prm.pool, 0, sizeof(PoolControl), ctx->stream));
+    if (again)
+      CK(cudaMemsetAsync(prm.pool, 0, sizeof(PoolControl), ctx->stream));
   }
   const int out_list = pass & 1;
   prm.overflow = out_list ? ctx->d_ovf1.p : ctx->d_ovf0.p;
   prm.overflow_count = cnt + (out_list ? C_OVF1 : C_OVF0);
-  CK(cudaMemsetAsync(prm.overflow_count, 0, sizeof(unsigned long long), ctx->stream));
+  if (again)
+    CK(cudaMemsetAsync(prm.overflow_count, 0, sizeof(unsigned long long), ctx->stream));
   if (pass > 0)
   {
     prm.in_records = out_list ? ctx->d_ovf0.p : ctx->d_ovf1.p;
@@ -511,20 +553,15 @@ mtg_destroy(mtg_ctx * ctx)
   if (!ctx)
     return MTG_OK;
   cudaSetDevice(ctx->device);
-  DevBuf * bufs[] = {&ctx->d_sims,   &ctx->d_order, &ctx->d_order_end, &ctx->d_species, &ctx->d_mats,    &ctx->d_row_species,
-                     &ctx->d_stop,   &ctx->p_vac,      &ctx->p_coll,    &ctx->p_eel,     &ctx->p_enuc,
-                     &ctx->p_fx,     &ctx->p_fy,       &ctx->p_fz,      &ctx->p_state,   &ctx->d_totals,
-                     &ctx->d_hist,   &ctx->d_err,      &ctx->d_counters, &ctx->d_stacks, &ctx->d_ovf0,
-                     &ctx->d_ovf1,   &ctx->d_records,  &ctx->d_events,  &ctx->d_jobs,    &ctx->d_job_first,
-                     &ctx->d_partials,
-                     &ctx->d_out,    &ctx->d_tmp0,     &ctx->d_tmp1,    &ctx->d_tmp2,    &ctx->d_tmp3,
-                     &ctx->d_mats32, &ctx->d_cold32, &ctx->d_sims32, &ctx->d_sg_params, &ctx->d_sg_net,
-                     &ctx->d_vox,    &ctx->d_vox_range, &ctx->d_vox_sum, &ctx->d_vox_part, &ctx->d_cl, &ctx->d_cl32,
-                     &ctx->d_cl_next, &ctx->d_cl_head, &ctx->d_cl_mask, &ctx->d_pool_ctl, &ctx->d_pool_ring,
-                     &ctx->d_pool_box, &ctx->d_pool_recs};
+  DevBuf * bufs[] = {&ctx->d_tables,   &ctx->d_run,       &ctx->d_stop,      &ctx->d_stacks,    &ctx->d_ovf0,
+                     &ctx->d_ovf1,     &ctx->d_records,   &ctx->d_events,    &ctx->d_partials,  &ctx->d_tmp0,
+                     &ctx->d_tmp1,     &ctx->d_tmp2,      &ctx->d_tmp3,      &ctx->d_sg_params, &ctx->d_sg_net,
+                     &ctx->d_vox,      &ctx->d_vox_part,  &ctx->d_pool_ring, &ctx->d_pool_box,  &ctx->d_pool_recs};
   for (DevBuf * b : bufs)
     if (b->p)
       cudaFree(b->p);
+  if (ctx->h_results)
+    cudaFreeHost(ctx->h_results);
   for (auto & e : ctx->ev)
     if (e)
       cudaEventDestroy(e);
@@ -603,62 +640,38 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
   const HostTables & t = ctx->tables;
   const size_t ns = t.sims.size();
   const size_t np = size_t(std::max<long long>(t.total_primaries, 1));
-  CK(ensure(ctx->d_sims, sizeof(SimDesc) * ns));
-  CK(ensure(ctx->d_order, sizeof(int) * ns));
-  CK(ensure(ctx->d_order_end, sizeof(long long) * ns));
-  CK(ensure(ctx->d_species, sizeof(SpeciesConst) * t.species.size()));
-  CK(ensure(ctx->d_mats, sizeof(MatConst) * t.mats.size()));
-  CK(ensure(ctx->p_vac, 8 * np));
-  CK(ensure(ctx->p_coll, 8 * np));
-  CK(ensure(ctx->p_eel, 8 * np));
-  CK(ensure(ctx->p_enuc, 8 * np));
-  CK(ensure(ctx->p_fx, 8 * np));
-  CK(ensure(ctx->p_fy, 8 * np));
-  CK(ensure(ctx->p_fz, 8 * np));
-  CK(ensure(ctx->p_state, 4 * np));
-  CK(ensure(ctx->d_totals, sizeof(SimTotals) * ns));
-  CK(ensure(ctx->d_hist, 8 * size_t(std::max<long long>(t.hist_total, 1))));
-  CK(ensure(ctx->d_err, 16));
-  CK(ensure(ctx->d_counters, 8 * C_COUNT));
-  if (t.voxel_total > 0)
+  const bool fp64 = ctx->cfg.precision == MTG_PREC_FP64;
+  const bool clusters = !t.clusters.empty() || !t.cl_head.empty();
+  const bool voxels = t.voxel_total > 0;
+
+  // the run's results first (collect copies them together), then what else a run clears
+  ctx->prepared = ctx->launched = false;
+  CK(cut(ctx->d_run, {{&ctx->d_counters, 8 * C_COUNT},
+                      {&ctx->d_err, 16},
+                      {&ctx->d_totals, sizeof(SimTotals) * ns},
+                      {&ctx->d_out, sizeof(double) * NQ * ns},
+                      {&ctx->d_vox_sum, sizeof(double) * ns},
+                      {&ctx->d_hist, 8 * size_t(std::max<long long>(t.hist_total, 1))},
+                      {&ctx->d_pool_ctl, ctx->cfg.precision != MTG_PREC_FP32 ? sizeof(PoolControl) * MAX_PASSES : 16},
+                      {&ctx->p_vac, 8 * np},
+                      {&ctx->p_coll, 8 * np},
+                      {&ctx->p_eel, 8 * np},
+                      {&ctx->p_enuc, 8 * np},
+                      {&ctx->p_state, 4 * np},
+                      {&ctx->p_fx, 8 * np},
+                      {&ctx->p_fy, 8 * np},
+                      {&ctx->p_fz, 8 * np}}));
+
+  ctx->results_bytes = size_t(static_cast<char *>(ctx->d_hist.p) - static_cast<char *>(ctx->d_run.p));
+  if (ctx->h_bytes < ctx->results_bytes)
   {
-    std::vector<long long> vr(2 * ns);
-    for (size_t s = 0; s < ns; ++s)
-    {
-      const SimDesc & d = t.sims[s];
-      vr[2 * s] = d.voxel_base;
-      vr[2 * s + 1] = d.voxel_n[0] > 0 ? (long long)d.voxel_n[0] * d.voxel_n[1] * d.voxel_n[2] : 0;
-    }
-    CK(ensure(ctx->d_vox, sizeof(double) * size_t(t.voxel_total)));
-    CK(ensure(ctx->d_vox_range, sizeof(long long) * vr.size()));
-    CK(ensure(ctx->d_vox_sum, sizeof(double) * ns));
-    CK(ensure(ctx->d_vox_part, voxel_partials_bytes(int(ns))));
-    CK(h2d(ctx, ctx->d_vox_range.p, vr.data(), sizeof(long long) * vr.size()));
+    if (ctx->h_results)
+      cudaFreeHost(ctx->h_results);
+    ctx->h_results = nullptr;
+    ctx->h_bytes = 0;
+    CK(cudaMallocHost(&ctx->h_results, ctx->results_bytes));
+    ctx->h_bytes = ctx->results_bytes;
   }
-  // cluster samples: the cluster arrays, and the simulations pointing at them
-  ctx->sims_dev = t.sims;
-  if (!t.clusters.empty() || !t.cl_head.empty())
-  {
-    CK(ensure(ctx->d_cl, sizeof(Cl4d) * std::max<size_t>(t.clusters.size(), 1)));
-    CK(ensure(ctx->d_cl_next, sizeof(int) * std::max<size_t>(t.cl_next.size(), 1)));
-    CK(ensure(ctx->d_cl_head, sizeof(int) * std::max<size_t>(t.cl_head.size(), 1)));
-    if (!t.clusters.empty())
-    {
-      CK(h2d(ctx, ctx->d_cl.p, t.clusters.data(), sizeof(Cl4d) * t.clusters.size()));
-      CK(h2d(ctx, ctx->d_cl_next.p, t.cl_next.data(), sizeof(int) * t.cl_next.size()));
-    }
-    CK(h2d(ctx, ctx->d_cl_head.p, t.cl_head.data(), sizeof(int) * t.cl_head.size()));
-    CK(ensure(ctx->d_cl_mask, sizeof(uint32_t) * std::max<size_t>(t.cl_mask.size(), 1)));
-    if (!t.cl_mask.empty())
-      CK(h2d(ctx, ctx->d_cl_mask.p, t.cl_mask.data(), sizeof(uint32_t) * t.cl_mask.size()));
-    patch_cluster_pointers(ctx->sims_dev, ptr<Cl4d>(ctx->d_cl), ptr<int>(ctx->d_cl_next), ptr<int>(ctx->d_cl_head),
-                           ptr<uint32_t>(ctx->d_cl_mask));
-  }
-  CK(h2d(ctx, ctx->d_sims.p, ctx->sims_dev.data(), sizeof(SimDesc) * ns));
-  CK(h2d(ctx, ctx->d_order.p, t.order.data(), sizeof(int) * ns));
-  CK(h2d(ctx, ctx->d_order_end.p, t.order_end.data(), sizeof(long long) * ns));
-  CK(h2d(ctx, ctx->d_species.p, t.species.data(), sizeof(SpeciesConst) * t.species.size()));
-  CK(h2d(ctx, ctx->d_mats.p, t.mats.data(), sizeof(MatConst) * t.mats.size()));
 
   // reduction jobs: contiguous chunks of each simulation's primaries
   ctx->jobs.clear();
@@ -671,57 +684,106 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
       ctx->jobs.push_back(ReduceJob{int(s), b + o, b + std::min(n, o + chunk)});
     ctx->job_first.push_back(int(ctx->jobs.size()));
   }
-  CK(ensure(ctx->d_jobs, sizeof(ReduceJob) * std::max<size_t>(ctx->jobs.size(), 1)));
-  CK(ensure(ctx->d_job_first, sizeof(int) * ctx->job_first.size()));
   CK(ensure(ctx->d_partials, sizeof(double) * NQ * std::max<size_t>(ctx->jobs.size(), 1)));
-  CK(ensure(ctx->d_out, sizeof(double) * NQ * ns));
-  if (!ctx->jobs.empty())
-    CK(h2d(ctx, ctx->d_jobs.p, ctx->jobs.data(), sizeof(ReduceJob) * ctx->jobs.size()));
-  CK(h2d(ctx, ctx->d_job_first.p, ctx->job_first.data(), sizeof(int) * ctx->job_first.size()));
-
-  if (ctx->cfg.precision != MTG_PREC_FP64)
+  std::vector<long long> vr;
+  if (voxels)
+  {
+    vr.resize(2 * ns);
+    for (size_t s = 0; s < ns; ++s)
+    {
+      const SimDesc & d = t.sims[s];
+      vr[2 * s] = d.voxel_base;
+      vr[2 * s + 1] = d.voxel_n[0] > 0 ? (long long)d.voxel_n[0] * d.voxel_n[1] * d.voxel_n[2] : 0;
+    }
+    CK(ensure(ctx->d_vox, sizeof(double) * size_t(t.voxel_total)));
+    CK(ensure(ctx->d_vox_part, voxel_partials_bytes(int(ns))));
+  }
+  // The FP64 engine takes all species and material rows.  The others take their
+  // single-precision copies, and the FP64 rows of each distinct (species, material) for
+  // the stopping tables only: in a batch of thousands of simulations a few of many.
+  const size_t nrows = t.stop_row_mat.size();
+  std::vector<SpeciesConst> row_species;
+  std::vector<MatConst> row_mats;
+  std::vector<Cl4f> c32;
+  if (!fp64)
+  {
+    for (size_t r = 0; r < nrows; ++r)
+    {
+      row_species.push_back(t.species[size_t(t.stop_row_species[r])]);
+      row_mats.push_back(t.mats[size_t(t.stop_row_mat[r])]);
+    }
+    build_fp32_tables(t, ctx->mc32, ctx->cold32, ctx->sm32);
+    for (const Cl4d & c : t.clusters)
+      c32.push_back(Cl4f{float(c.x), float(c.y), float(c.z), float(c.r)});
+    CK(ensure(ctx->d_stop, 2 * sizeof(float) * STOP_N * nrows)); // (S, p_max) pairs
+  }
+  ctx->sims_dev = t.sims;
+  struct Table
+  {
+    DevBuf * b;
+    const void * src;
+    size_t bytes;
+  };
+  const std::vector<SpeciesConst> & species = fp64 ? t.species : row_species;
+  const std::vector<MatConst> & mats = fp64 ? t.mats : row_mats;
+  const Table tables[] = {
+      {&ctx->d_sims, ctx->sims_dev.data(), sizeof(SimDesc) * ns},
+      {&ctx->d_order, t.order.data(), sizeof(int) * ns},
+      {&ctx->d_order_end, t.order_end.data(), sizeof(long long) * ns},
+      {&ctx->d_species, species.data(), sizeof(SpeciesConst) * species.size()},
+      {&ctx->d_mats, mats.data(), sizeof(MatConst) * mats.size()},
+      {&ctx->d_jobs, ctx->jobs.data(), sizeof(ReduceJob) * ctx->jobs.size()},
+      {&ctx->d_job_first, ctx->job_first.data(), sizeof(int) * ctx->job_first.size()},
+      {&ctx->d_vox_range, vr.data(), sizeof(long long) * vr.size()},
+      {&ctx->d_cl, t.clusters.data(), sizeof(Cl4d) * t.clusters.size()},
+      {&ctx->d_cl_next, t.cl_next.data(), sizeof(int) * t.cl_next.size()},
+      {&ctx->d_cl_head, t.cl_head.data(), sizeof(int) * t.cl_head.size()},
+      {&ctx->d_cl_mask, t.cl_mask.data(), sizeof(uint32_t) * t.cl_mask.size()},
+      {&ctx->d_cl32, c32.data(), sizeof(Cl4f) * c32.size()},
+      {&ctx->d_mats32, ctx->mc32.data(), fp64 ? 0 : sizeof(Mat32) * ctx->mc32.size()},
+      {&ctx->d_cold32, ctx->cold32.data(), fp64 ? 0 : sizeof(MatCold32) * ctx->cold32.size()},
+      {&ctx->d_sims32, ctx->sm32.data(), fp64 ? 0 : sizeof(Sim32) * ctx->sm32.size()},
+  };
+  std::vector<Cut> cuts;
+  size_t staged = 0;
+  for (const Table & x : tables)
+  {
+    cuts.push_back({x.b, x.bytes});
+    staged += aligned(x.bytes);
+  }
+  CK(cut(ctx->d_tables, cuts));
+  // cluster samples: the simulations point at the cluster arrays
+  if (clusters)
+  {
+    patch_cluster_pointers(ctx->sims_dev, ptr<Cl4d>(ctx->d_cl), ptr<int>(ctx->d_cl_next), ptr<int>(ctx->d_cl_head),
+                           ptr<uint32_t>(ctx->d_cl_mask));
+    if (!fp64)
+      for (size_t i = 0; i < ctx->sm32.size(); ++i)
+        if (ctx->sm32[i].geometry == 1)
+        {
+          Sim32 & d = ctx->sm32[i];
+          d.cl = ptr<Cl4f>(ctx->d_cl32) + t.sims[i].cl_base;
+          d.cl_next = ptr<int>(ctx->d_cl_next) + t.sims[i].cl_base;
+          d.cl_head = ptr<int>(ctx->d_cl_head) + t.sims[i].cell_base;
+          d.cl_mask = ptr<uint32_t>(ctx->d_cl_mask) + t.sims[i].mask_base;
+        }
+  }
+  ctx->staging.resize(staged);
+  size_t at = 0;
+  for (const Table & x : tables)
+  {
+    if (x.bytes)
+      std::memcpy(ctx->staging.data() + at, x.src, x.bytes);
+    at += aligned(x.bytes);
+  }
+  CK(h2d(ctx, ctx->d_tables.p, ctx->staging.data(), staged));
+  if (!fp64)
   {
     // FP32 path: stopping tables evaluated on the device in FP64, one row per
     // distinct (species, material) of the run
-    const size_t nrows = t.stop_row_mat.size();
-    CK(ensure(ctx->d_row_species, 2 * sizeof(int) * nrows));
-    CK(ensure(ctx->d_stop, 2 * sizeof(float) * STOP_N * nrows)); // (S, p_max) pairs
-    int * d_row_species = ptr<int>(ctx->d_row_species);
-    int * d_row_mat = d_row_species + nrows;
-    CK(h2d(ctx, d_row_species, t.stop_row_species.data(), sizeof(int) * nrows));
-    CK(h2d(ctx, d_row_mat, t.stop_row_mat.data(), sizeof(int) * nrows));
     const double lo = std::log(STOP_EMIN), hi = std::log(t.emax * 1.05);
-    CK(launch_build_stop_tables(ptr<SpeciesConst>(ctx->d_species), ptr<MatConst>(ctx->d_mats), d_row_mat,
-                                int(nrows), d_row_species, ptr<float>(ctx->d_stop), lo, (hi - lo) / (STOP_N - 1),
-                                nullptr));
-    CK(cudaDeviceSynchronize());
-    std::vector<Mat32> & mc32 = ctx->mc32;
-    std::vector<Sim32> & sm32 = ctx->sm32;
-    build_fp32_tables(t, mc32, ctx->cold32, sm32);
-    if (!t.clusters.empty() || !t.cl_head.empty())
-    {
-      std::vector<Cl4f> c32(t.clusters.size());
-      for (size_t l = 0; l < c32.size(); ++l)
-        c32[l] = Cl4f{float(t.clusters[l].x), float(t.clusters[l].y), float(t.clusters[l].z),
-                      float(t.clusters[l].r)};
-      CK(ensure(ctx->d_cl32, sizeof(Cl4f) * std::max<size_t>(c32.size(), 1)));
-      if (!c32.empty())
-        CK(h2d(ctx, ctx->d_cl32.p, c32.data(), sizeof(Cl4f) * c32.size()));
-      for (size_t i = 0; i < sm32.size(); ++i)
-        if (sm32[i].geometry == 1)
-        {
-          sm32[i].cl = ptr<Cl4f>(ctx->d_cl32) + t.sims[i].cl_base;
-          sm32[i].cl_next = ptr<int>(ctx->d_cl_next) + t.sims[i].cl_base;
-          sm32[i].cl_head = ptr<int>(ctx->d_cl_head) + t.sims[i].cell_base;
-          sm32[i].cl_mask = ptr<uint32_t>(ctx->d_cl_mask) + t.sims[i].mask_base;
-        }
-    }
-    CK(ensure(ctx->d_mats32, sizeof(Mat32) * mc32.size()));
-    CK(ensure(ctx->d_cold32, sizeof(MatCold32) * ctx->cold32.size()));
-    CK(ensure(ctx->d_sims32, sizeof(Sim32) * sm32.size()));
-    CK(h2d(ctx, ctx->d_mats32.p, mc32.data(), sizeof(Mat32) * mc32.size()));
-    CK(h2d(ctx, ctx->d_cold32.p, ctx->cold32.data(), sizeof(MatCold32) * ctx->cold32.size()));
-    CK(h2d(ctx, ctx->d_sims32.p, sm32.data(), sizeof(Sim32) * sm32.size()));
+    CK(launch_build_stop_tables(ptr<SpeciesConst>(ctx->d_species), ptr<MatConst>(ctx->d_mats), nullptr, int(nrows),
+                                nullptr, ptr<float>(ctx->d_stop), lo, (hi - lo) / (STOP_N - 1), nullptr));
   }
   if (ctx->record_cap > 0)
     CK(ensure(ctx->d_records, sizeof(MemberRecord) * size_t(ctx->record_cap)));
@@ -730,6 +792,7 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
   st = setup_launch_shape(ctx);
   if (st != MTG_OK)
     return st;
+  CK(cudaDeviceSynchronize()); // the tables are in place for a launch on any stream
   ctx->prepared = true;
   ctx->launched = false;
   return MTG_OK;
@@ -745,21 +808,13 @@ mtg_launch_async(mtg_ctx * ctx, void * stream)
     return fail(ctx, MTG_ERR_STATE, "mtg_prepare must come first");
   ctx->stream = reinterpret_cast<cudaStream_t>(stream);
   const HostTables & t = ctx->tables;
-  const size_t np = size_t(std::max<long long>(t.total_primaries, 1));
   ctx->stats.launches = 0;
   ctx->stats.drains = 0;
   cudaStream_t s = ctx->stream;
-  CK(cudaMemsetAsync(ctx->p_vac.p, 0, 8 * np, s));
-  CK(cudaMemsetAsync(ctx->p_coll.p, 0, 8 * np, s));
-  CK(cudaMemsetAsync(ctx->p_eel.p, 0, 8 * np, s));
-  CK(cudaMemsetAsync(ctx->p_enuc.p, 0, 8 * np, s));
-  CK(cudaMemsetAsync(ctx->p_state.p, 0, 4 * np, s));
-  CK(cudaMemsetAsync(ctx->d_totals.p, 0, sizeof(SimTotals) * t.sims.size(), s));
-  CK(cudaMemsetAsync(ctx->d_hist.p, 0, 8 * size_t(std::max<long long>(t.hist_total, 1)), s));
-  CK(cudaMemsetAsync(ctx->d_err.p, 0, 16, s));
+  // counters, totals, histograms and the primaries' tallies (all of d_run before p_fx)
+  CK(cudaMemsetAsync(ctx->d_run.p, 0, size_t(static_cast<char *>(ctx->p_fx.p) - static_cast<char *>(ctx->d_run.p)), s));
   if (t.voxel_total > 0)
     CK(cudaMemsetAsync(ctx->d_vox.p, 0, sizeof(double) * size_t(t.voxel_total), s));
-  CK(cudaMemsetAsync(ctx->d_counters.p, 0, 8 * C_COUNT, s));
   CK(cudaEventRecord(ctx->ev[0], s));
   st = launch_pass(ctx, 0);
   if (st != MTG_OK)
@@ -822,12 +877,24 @@ static mtg_status
 collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
 {
   mtg_status st = MTG_OK;
-  CK(cudaStreamSynchronize(ctx->stream));
   const HostTables & t = ctx->tables;
-  unsigned long long cnt[C_COUNT];
-  ctx->stats.d2h_bytes = sizeof cnt + sizeof(unsigned int) + (long long)(sizeof(double) * NQ + sizeof(SimTotals)) *
-                         (long long)t.sims.size() + (hist ? 8LL * t.hist_total : 0LL);
-  CK(cudaMemcpy(cnt, ctx->d_counters.p, sizeof cnt, cudaMemcpyDeviceToHost));
+  const size_t ns = t.sims.size();
+  // everything but the histograms in one copy
+  auto fetch = [&]() {
+    const cudaError_t e = cudaMemcpyAsync(ctx->h_results, ctx->d_run.p, ctx->results_bytes, cudaMemcpyDeviceToHost,
+                                          ctx->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(ctx->stream);
+  };
+  auto result = [&](const DevBuf & b) {
+    return ctx->h_results + (static_cast<char *>(b.p) - static_cast<char *>(ctx->d_run.p));
+  };
+  const unsigned long long * cnt = reinterpret_cast<const unsigned long long *>(result(ctx->d_counters));
+  const unsigned int & errf = *reinterpret_cast<const unsigned int *>(result(ctx->d_err));
+  const SimTotals * tot = reinterpret_cast<const SimTotals *>(result(ctx->d_totals));
+  const double * out = reinterpret_cast<const double *>(result(ctx->d_out));
+  const double * vsum = reinterpret_cast<const double *>(result(ctx->d_vox_sum));
+  ctx->stats.d2h_bytes = (long long)ctx->results_bytes + (hist ? 8LL * t.hist_total : 0LL);
+  CK(fetch());
   // further drain passes while the last pass spilled members
   long long overflowed = (long long)cnt[C_OVF0];
   int extra = 0;
@@ -838,26 +905,21 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
     if (st != MTG_OK)
       return st;
     ++extra;
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaMemcpy(cnt, ctx->d_counters.p, sizeof cnt, cudaMemcpyDeviceToHost));
+    CK(fetch());
   }
   const bool unfinished = cnt[ctx->ovf_last ? C_OVF1 : C_OVF0] > 0;
   // an overflow list that filled dropped members: the run is made again with lists
   // four times larger, kept for later runs.  The random draws depend on the members'
   // keys, not on the schedule, so the repeated run is the run the larger lists would
   // have given in the first place.
+  if ((errf & ERRB_QUEUE_FULL) && retry < MAX_OVF_RETRIES && grow_overflow(ctx, ctx->ovf_cap * 4))
   {
-    unsigned int errq = 0;
-    CK(cudaMemcpy(&errq, ctx->d_err.p, sizeof errq, cudaMemcpyDeviceToHost));
-    if ((errq & ERRB_QUEUE_FULL) && retry < MAX_OVF_RETRIES && grow_overflow(ctx, ctx->ovf_cap * 4))
-    {
-      const int launched_before = ctx->stats.launches; // the count covers every attempt
-      st = mtg_launch_async(ctx, ctx->stream);
-      if (st != MTG_OK)
-        return st;
-      ctx->stats.launches += launched_before;
-      return collect_run(ctx, totals, hist, retry + 1);
-    }
+    const int launched_before = ctx->stats.launches; // the count covers every attempt
+    st = mtg_launch_async(ctx, ctx->stream);
+    if (st != MTG_OK)
+      return st;
+    ctx->stats.launches += launched_before;
+    return collect_run(ctx, totals, hist, retry + 1);
   }
   if (extra)
   {
@@ -866,7 +928,10 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
     if (st != MTG_OK)
       return st;
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    if (t.voxel_total > 0)
+      CK(launch_voxel_sum(ptr<double>(ctx->d_vox), ptr<long long>(ctx->d_vox_range), int(ns),
+                          ptr<double>(ctx->d_vox_part), ptr<double>(ctx->d_vox_sum), ctx->stream));
+    CK(fetch());
   }
   // with extra drain passes the kernel time runs to the end of the last one (it
   // includes the first reduction and the host's turnaround between the passes)
@@ -884,31 +949,13 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
   ctx->stats.overflowed = overflowed;
 
   ctx->stats.events_overflowed = 0;
-  unsigned int errf = 0;
-  CK(cudaMemcpy(&errf, ctx->d_err.p, sizeof errf, cudaMemcpyDeviceToHost));
-  const size_t ns = t.sims.size();
-  std::vector<double> out(NQ * ns);
-  std::vector<SimTotals> tot(ns);
-  CK(cudaMemcpy(out.data(), ctx->d_out.p, sizeof(double) * NQ * ns, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(tot.data(), ctx->d_totals.p, sizeof(SimTotals) * ns, cudaMemcpyDeviceToHost));
-  std::vector<double> vsum(ns, 0.0);
-  if (t.voxel_total > 0)
-  {
-    if (extra)
-    {
-      CK(launch_voxel_sum(ptr<double>(ctx->d_vox), ptr<long long>(ctx->d_vox_range), int(ns),
-                          ptr<double>(ctx->d_vox_part), ptr<double>(ctx->d_vox_sum), ctx->stream));
-      CK(cudaStreamSynchronize(ctx->stream));
-    }
-    CK(cudaMemcpy(vsum.data(), ctx->d_vox_sum.p, sizeof(double) * ns, cudaMemcpyDeviceToHost));
-  }
   long long coll_all = 0;
   if (totals)
     for (size_t s = 0; s < ns; ++s)
     {
       mtg_totals & o = totals[s];
       std::memset(&o, 0, sizeof o);
-      const double * q = &out[NQ * s];
+      const double * q = out + NQ * s;
       o.primaries = t.sims[s].n_primaries;
       o.members = (long long)tot[s].members;
       o.collisions = (long long)llround(q[2]);
@@ -943,22 +990,13 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
       coll_all += o.collisions;
     }
   ctx->stats.collisions = coll_all;
+  static_assert(sizeof(long long) == sizeof(unsigned long long), "histogram counts are copied as they are");
   if (hist && t.hist_total > 0)
-  {
-    std::vector<unsigned long long> h(t.hist_total);
-    CK(cudaMemcpy(h.data(), ctx->d_hist.p, 8 * h.size(), cudaMemcpyDeviceToHost));
-    for (long long i = 0; i < t.hist_total; ++i)
-      hist[i] = (long long)h[i];
-  }
+    CK(cudaMemcpy(hist, ctx->d_hist.p, 8 * size_t(t.hist_total), cudaMemcpyDeviceToHost));
   size_t bytes = 0;
-  DevBuf * bufs[] = {&ctx->d_sims,   &ctx->d_order, &ctx->d_order_end, &ctx->d_species, &ctx->d_mats,    &ctx->d_row_species,
-                     &ctx->d_stop,   &ctx->p_vac,      &ctx->p_coll,    &ctx->p_eel,     &ctx->p_enuc,
-                     &ctx->p_fx,     &ctx->p_fy,       &ctx->p_fz,      &ctx->p_state,   &ctx->d_totals,
-                     &ctx->d_hist,   &ctx->d_err,      &ctx->d_counters, &ctx->d_stacks, &ctx->d_ovf0,
-                     &ctx->d_ovf1,   &ctx->d_records,  &ctx->d_events,  &ctx->d_jobs,    &ctx->d_job_first,
-                     &ctx->d_partials,
-                     &ctx->d_out,    &ctx->d_mats32, &ctx->d_cold32, &ctx->d_sims32, &ctx->d_vox, &ctx->d_vox_part,
-                     &ctx->d_pool_ctl, &ctx->d_pool_ring, &ctx->d_pool_box, &ctx->d_pool_recs};
+  DevBuf * bufs[] = {&ctx->d_tables,  &ctx->d_run,      &ctx->d_stop,      &ctx->d_stacks,   &ctx->d_ovf0,
+                     &ctx->d_ovf1,    &ctx->d_records,  &ctx->d_events,    &ctx->d_partials, &ctx->d_vox,
+                     &ctx->d_vox_part, &ctx->d_pool_ring, &ctx->d_pool_box, &ctx->d_pool_recs};
   for (DevBuf * b : bufs)
     bytes += b->bytes;
   ctx->stats.device_bytes = bytes;

@@ -230,7 +230,7 @@ build_stop_tables_kernel(const SpeciesConst * species, const MatConst * mats, co
   const MatConst & mc = mats[row_mat ? row_mat[row] : row];
   const double eeg = sqrt(E * mc.f * mc.epsdg);
   const double pmax = mc.a / (eeg + sqrt(eeg) + 0.125 * pow64(eeg, 0.1));
-  out[2 * i] = float(material_stop64(species[row_species[row]], mc, E));
+  out[2 * i] = float(material_stop64(species[row_species ? row_species[row] : row], mc, E));
   out[2 * i + 1] = float(pmax);
 }
 

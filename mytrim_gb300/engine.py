@@ -160,6 +160,7 @@ class _SimRow(C.Structure):
     _fields_ = [(n, _SampleRow if n == "sample" else t) for n, t in F.Sim._fields_]
 
 
+_TOTALS_DTYPE = np.dtype(F.Totals)
 _SIM_DTYPE = np.dtype(_SimRow)
 assert _SIM_DTYPE.itemsize == C.sizeof(F.Sim)
 _NO_MATERIAL = bytes(C.sizeof(F.Material))
@@ -354,26 +355,29 @@ class Engine:
         (complete) tallies; stats()["events_overflowed"] then reads 1."""
         n = len(self._sims)
         tot = (F.Totals * n)()
-        nh = sum(sum(s.hist_sizes()) for s in self._sims)
-        hist = (C.c_longlong * max(nh, 1))()
-        st = self.lib.mtg_collect(self.ctx, tot, hist)
+        sizes = [s.hist_sizes() for s in self._sims]
+        nh = sum(map(sum, sizes))
+        h = np.zeros(max(nh, 1), dtype=np.int64)
+        st = self.lib.mtg_collect(self.ctx, tot, h.ctypes.data_as(C.POINTER(C.c_longlong)))
         if check and not (allow_event_overflow and st == F.ERR_QUEUE_FULL and self.stats()["events_overflowed"]):
             self._check(st)
         out = []
-        off = 0
-        rows = np.ctypeslib.as_array(tot).tolist()
-        names = F.Totals.field_names()
-        h = np.frombuffer(hist, dtype=np.int64, count=max(nh, 1))
-        for i, s in enumerate(self._sims):
-            d = dict(zip(names, rows[i]))
-            hr, hv, hp, hl, he = s.hist_sizes()
-            d["hist_range"] = h[off:off + hr].copy()
-            d["hist_vac"] = h[off + hr:off + hr + hv].copy()
-            d["hist_repl"] = h[off + hr + hv:off + hr + hv + hp].copy()
-            o = off + hr + hv + hp
-            d["hist_lateral"] = h[o:o + hl].copy().reshape(s.hist_lateral_n, s.hist_lateral_n)
-            d["hist_evac"] = h[o + hl:o + hl + he].copy().reshape(s.hist_evac_rows if he else 0, hv if he else 0)
-            off += hr + hv + hp + hl + he
+        rows = np.frombuffer(tot, dtype=_TOTALS_DTYPE, count=n).tolist()
+        names = _TOTALS_DTYPE.names
+        at = 0
+
+        def take(k):
+            nonlocal at
+            at += k
+            return h[at - k:at].copy() if k else np.empty(0, dtype=np.int64)
+
+        for s, row, (hr, hv, hp, hl, he) in zip(self._sims, rows, sizes):
+            d = dict(zip(names, row))
+            d["hist_range"] = take(hr)
+            d["hist_vac"] = take(hv)
+            d["hist_repl"] = take(hp)
+            d["hist_lateral"] = take(hl).reshape(s.hist_lateral_n, s.hist_lateral_n)
+            d["hist_evac"] = take(he).reshape(s.hist_evac_rows if he else 0, hv if he else 0)
             d["status"] = st
             out.append(d)
         return out
