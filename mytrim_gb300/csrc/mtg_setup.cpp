@@ -269,10 +269,7 @@ build_fp32_tables(const HostTables & t, std::vector<Mat32> & mats, std::vector<M
     Sim32 & o = sims[i];
     std::memset(&o, 0, sizeof o);
     for (int k = 0; k < MAX_LAYERS; ++k)
-    {
-      o.layer_end[k] = float(d.layer_end[k]);
-      o.layer_mat[k] = d.layer_mat[k];
-    }
+      o.layer_end[k] = float(d.layer_end[k]); // layer k is of material k
     for (int k = 0; k < 3; ++k)
     {
       o.w[k] = float(d.w[k]);
@@ -284,15 +281,8 @@ build_fp32_tables(const HostTables & t, std::vector<Mat32> & mats, std::vector<M
     o.n_layers = d.n_layers;
     o.n_mat = d.n_mat;
     o.mat_base = d.mat_base;
-    o.species_base = d.species_base;
     o.Ef = float(d.Ef);
-    o.flscale = float(d.invscale);
-    o.tau = float(d.tau);
-    o.cw = float(d.cw);
-    o.range_mode = d.range_mode;
-    o.primaries_only = d.primaries_only;
     o.follow_gen = d.follow_gen;
-    o.kp_gen = d.kp_gen;
     o.potential = d.potential;
     o.geometry = d.geometry;
     o.n_clusters = d.n_clusters;

@@ -240,17 +240,17 @@ stage_net_offset(int n_mats)
   return sizeof(Mat32) * size_t(n_mats);
 }
 
-struct Sim32
+struct alignas(16) Sim32
 {
   float layer_end[MAX_LAYERS];
-  int layer_mat[MAX_LAYERS];
+  // what every collision reads, in 16-byte pieces
+  int n_layers, n_mat, mat_base, any_cut;
+  float Ef;
+  int follow_gen, geometry, potential;
+  float cut_lo[3], cut_hi[3]; // where a CUT boundary takes members out; infinities on other axes
+  float pad[2];
   float w[3];
   int bc[3];
-  int n_layers, n_mat, mat_base, species_base;
-  float Ef, flscale, tau, cw; // flscale = 1 / length scale
-  int range_mode, primaries_only, any_cut, geometry;
-  float cut_lo[3], cut_hi[3]; // where a CUT boundary takes members out; infinities on other axes
-  int follow_gen, kp_gen, potential, pad1;
   // sampleClusters geometry (see SimDesc)
   int kn[3];
   int n_clusters;
