@@ -11,8 +11,10 @@
 //     counter (one atomicAdd per warp refill);
 //   * recoils are pushed with a ballot + prefix count; a full stack spills into
 //     a global overflow list that a follow-up launch drains.
-// No warp ever waits on another, so the kernel needs no spin loops; every loop
-// is bounded (collisions per member, Newton iterations, rejection passes).
+// In the FP64 and surrogate kernels a busy warp sends recoils to warps that have run
+// out (RecoilPool); the only wait in them is an idle warp's, for 20 ms at most.  Every
+// loop is bounded (collisions per member, Newton iterations, rejection passes).  The
+// single-precision kernel is in mtg_cascade32.cuh; it shares the tallies and parameters.
 //
 // Random numbers are keyed by the member's path key and collision index, so the
 // result does not depend on which lane or warp ran which member.
@@ -357,7 +359,7 @@ widen_f32(float f)
 }
 
 // Plain FP32 accumulator for the per-collision energy sums of the FP32 engine;
-// the engine hands it to the FP64 per-primary arrays every 64 collisions
+// the engine hands it to the FP64 per-primary arrays every 64 iterations
 // (LaneSink::hand_over), so each float sum stays short and accurate to ~1e-7
 struct AccF32
 {
