@@ -236,7 +236,8 @@ typedef struct
   double reduce_ms;        /* device time of the tally reduction of the last run */
   int launches;            /* kernels launched by the last run */
   int drains;              /* overflow drain passes of the last run */
-  int grid, block;         /* cascade launch shape */
+  int grid, block;         /* cascade launch shape (runs of fewer primaries than warps
+                              launch fewer blocks) */
   int stack_capacity;
   long long overflowed;    /* members spilled to the overflow list */
   long long collisions;
