@@ -425,7 +425,7 @@ struct Blocks32
       SURROGATE ? 4 : LVL == LVL_LEAN || LVL == LVL_MID || LVL == LVL_EVENTS ? 8 : 7;
 };
 
-template <int LVL, bool SURROGATE, bool ONE>
+template <int LVL, bool SURROGATE, bool ONE, bool PACED = false>
 __global__ void __launch_bounds__(128, Blocks32<LVL, SURROGATE>::value)
 cascade32_kernel(const __grid_constant__ EngineParams prm, const __grid_constant__ Tables32 tabs,
                  const __grid_constant__ One32 one)
@@ -507,6 +507,7 @@ cascade32_kernel(const __grid_constant__ EngineParams prm, const __grid_constant
   [[maybe_unused]] RecoilPool<Rec> pool;
   [[maybe_unused]] bool give = false;
   unsigned int steps = 0;
+  [[maybe_unused]] unsigned int take_mask = 2u * prm.take_mask + 1u; // halved at the first refill
 again:
   while (true)
   {
@@ -520,7 +521,11 @@ again:
       __syncwarp(); // the recoils other lanes pushed
       const int rank = __popc(idle & lt);
       const int npop = nidle < top ? nidle : top;
-      const int need = min(nidle - npop, max_take);
+      // PACED: a warp that has members takes new work in every (take_mask + 1)th iteration
+      // only; where it runs out in between, its cascades are smaller than was thought
+      if (PACED && idle == FULL)
+        take_mask >>= 1;
+      const int need = PACED && (steps & take_mask) && idle != FULL ? 0 : min(nidle - npop, max_take);
       long long base = 0;
       if (need > 0 && !work_done)
       {

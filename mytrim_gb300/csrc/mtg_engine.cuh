@@ -89,6 +89,8 @@ struct EngineParams
   uint32_t k0, k1;
   unsigned int max_collisions; // per member
   int max_take;                // fresh primaries one warp takes per refill (load balance)
+  unsigned int take_mask;      // iterations between two refills with new work, less one (2^k - 1);
+                               // 0: no pace (FP32 engine)
   int refill_min;              // idle lanes a warp waits for before refilling them
   int cold_offset;             // byte offset of the per-thread LaneCold slots in dynamic shared memory
   // optional per-member records (replay checks)

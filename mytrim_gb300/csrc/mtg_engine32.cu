@@ -30,29 +30,32 @@ namespace mtg
 
 // calls f with the kernel of a feature level; the surrogate engine runs the cluster-only
 // levels in the geometry variants
-template <bool SG, bool ONE, class F>
+template <bool SG, bool ONE, bool PACED, class F>
 static cudaError_t
 with_kernel(int level, F f)
 {
   switch (level)
   {
-    case LVL_LEAN: return f(cascade32_kernel<LVL_LEAN, SG, ONE>);
-    case LVL_MID: return f(cascade32_kernel<LVL_MID, SG, ONE>);
-    case LVL_EVENTS: return f(cascade32_kernel<LVL_EVENTS, SG, ONE>);
-    case LVL_GEO: return f(cascade32_kernel<LVL_GEO, SG, ONE>);
-    case LVL_CLU: return f(cascade32_kernel<SG ? LVL_GEO : LVL_CLU, SG, ONE>);
-    case LVL_CLU_EV: return f(cascade32_kernel<SG ? LVL_FULL : LVL_CLU_EV, SG, ONE>);
-    default: return f(cascade32_kernel<LVL_FULL, SG, ONE>);
+    case LVL_LEAN: return f(cascade32_kernel<LVL_LEAN, SG, ONE, PACED>);
+    case LVL_MID: return f(cascade32_kernel<LVL_MID, SG, ONE, PACED>);
+    case LVL_EVENTS: return f(cascade32_kernel<LVL_EVENTS, SG, ONE, PACED>);
+    case LVL_GEO: return f(cascade32_kernel<LVL_GEO, SG, ONE, PACED>);
+    case LVL_CLU: return f(cascade32_kernel<SG ? LVL_GEO : LVL_CLU, SG, ONE, PACED>);
+    case LVL_CLU_EV: return f(cascade32_kernel<SG ? LVL_FULL : LVL_CLU_EV, SG, ONE, PACED>);
+    default: return f(cascade32_kernel<LVL_FULL, SG, ONE, PACED>);
   }
 }
 
+// paced: only in the plain engine's runs of one simulation (EngineParams::take_mask)
 template <class F>
 static cudaError_t
-with_kernel(int level, int surrogate, int one, F f)
+with_kernel(int level, int surrogate, int one, int paced, F f)
 {
   if (surrogate)
-    return one ? with_kernel<true, true>(level, f) : with_kernel<true, false>(level, f);
-  return one ? with_kernel<false, true>(level, f) : with_kernel<false, false>(level, f);
+    return one ? with_kernel<true, true, false>(level, f) : with_kernel<true, false, false>(level, f);
+  if (paced)
+    return with_kernel<false, true, true>(level, f);
+  return one ? with_kernel<false, true, false>(level, f) : with_kernel<false, false, false>(level, f);
 }
 
 cudaError_t
@@ -78,7 +81,7 @@ launch_cascade32(const EngineParams & prm, const Fp32Tables & t, int grid, int b
   }
   else
     memset(&one, 0, sizeof one);
-  return with_kernel(prm.level, surrogate, prm.stage_tables, [&](auto * kernel) {
+  return with_kernel(prm.level, surrogate, prm.stage_tables, prm.take_mask != 0u, [&](auto * kernel) {
     kernel<<<grid, block, smem, st>>>(prm, tabs, one);
     return cudaGetLastError();
   });
@@ -89,7 +92,7 @@ launch_cascade32(const EngineParams & prm, const Fp32Tables & t, int grid, int b
 cudaError_t
 occupancy32(int block, size_t smem, int * blocks_per_sm, int surrogate, int level, int one)
 {
-  return with_kernel(level, surrogate, one, [&](auto * kernel) {
+  auto query = [&](auto * kernel) {
     if (smem > 48 * 1024)
     {
       const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -97,7 +100,14 @@ occupancy32(int block, size_t smem, int * blocks_per_sm, int surrogate, int leve
         return e;
     }
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel, block, smem);
-  });
+  };
+  if (one && !surrogate)
+  {
+    const cudaError_t e = with_kernel(level, 0, 1, 1, query);
+    if (e != cudaSuccess)
+      return e;
+  }
+  return with_kernel(level, surrogate, one, 0, query);
 }
 
 // bytes the stacks and overflow lists hold per recoil: the larger of the two layouts
