@@ -688,7 +688,7 @@ again:
       int state = ST_MOVING;
       if (EXT && a.gone)
       {
-        --ic; // dropped without a collision (no checkPKAState)
+        --sink.a_coll; // dropped without a collision (no checkPKAState), which its record counts
         flags = CF_DONE;
       }
       else
