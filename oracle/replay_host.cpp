@@ -14,6 +14,7 @@
 // Checks of single pieces of the same code, for the tests:
 //   replay_host <tables> --stopping              "Z1 m1 rho n Z m t ...", then energies -> stopping (hex)
 //   replay_host <tables> --scatter [potential]   lines "eps b" -> sin^2(theta/2) (hex)
+//   replay_host <tables> --stopspecial          stopping at infinities, zeros, NaN: where it differs
 //   replay_host <tables> --mathcheck [n]         exp64 / log64 short routes vs full forms
 //   replay_host <tables> --eval exp|log|pow       lines of hex-float arguments -> results (hex)
 //   replay_host <tables> --philox                lines of six hex words -> Philox outputs
@@ -27,6 +28,8 @@
 
 #include <algorithm>
 #include <cinttypes>
+#include <cmath>
+#include <limits>
 #include <vector>
 
 using namespace mtg;
@@ -239,6 +242,46 @@ main(int argc, char ** argv)
     }
     printf("%lld %lld\n", checked, bad);
     return bad ? 1 : 0;
+  }
+  if (argc >= 3 && std::string(argv[2]) == "--stopspecial")
+  {
+    // the stopping at energies that are no ordinary numbers against the whole formula as
+    // it stands in the reference (material.C:134-281): Z1 Z2 e, got, want where they differ
+    const double inf = std::numeric_limits<double>::infinity();
+    const double energies[] = {std::nan(""), inf, -inf, 0.0, -0.0, -5.0, -1e9, 5e-324, -1e-320, 1e-310, 1e-200, 1.7e308};
+    for (int Z1 = 1; Z1 <= MTG_SCOEF_ROWS; ++Z1)
+      for (int Z2 = 1; Z2 <= MTG_SCOEF_ROWS; ++Z2)
+      {
+        const SpeciesConst sc = make_species(rows, Z1, rows[Z1 - 1].m1);
+        const StopPair sp = make_stop_pair(rows, sc, Z2);
+        for (double e : energies)
+        {
+          auto proton = [&](double x) {
+            const double pe = x > 25.0 ? x : 25.0;
+            double s = proton_stop64_above(sp, pe, log64(pe));
+            return x <= 25.0 ? s * pow64(x / 25.0, sp.velpwr) : s;
+          };
+          const double le = log64(e);
+          double want;
+          if (sc.branch == STOP_H)
+            want = proton(e);
+          else if (sc.branch == STOP_HEAVY)
+          {
+            double yr = reduced_velocity64(sc, sp, e);
+            yr = yr < sp.yrcut ? sp.yrcut : yr;
+            const double zf = corrected_charge64(sc, sp, zeta64(sc, sp, yr), le);
+            want = yr <= sp.yrcut ? sp.sp_eee * (zf * zf) * exp64(sp.power * (le - log64(sp.eee)))
+                                  : proton(e) * (zf * zf);
+          }
+          else
+            continue; // helium's energy is limited below before the proton formula
+          want *= 10.0;
+          const double got = ion_stop64(sc, sp, e, le);
+          if (double_to_bits(got) != double_to_bits(want) && !(std::isnan(got) && std::isnan(want)))
+            printf("%d %d %a %a %a\n", Z1, Z2, e, got, want);
+        }
+      }
+    return 0;
   }
   if (argc >= 4 && std::string(argv[2]) == "--stopcheck")
   {
