@@ -129,6 +129,7 @@ struct mtg_ctx
   DevBuf d_cl, d_cl32, d_cl_next, d_cl_head, d_cl_mask; // sampleClusters geometry
   std::vector<SimDesc> sims_dev;             // SimDesc copies with device cluster pointers
   bool sg_ready = false;
+  bool quad_ready = false; // the quadrature's tables are on the device
   DevBuf p_vac, p_coll, p_eel, p_enuc, p_fx, p_fy, p_fz, p_state;
   DevBuf d_pool_ctl, d_pool_ring, d_pool_box, d_pool_recs; // recoils shared between warps (RecoilPool)
   unsigned int pool_nonce = 0;
@@ -542,6 +543,15 @@ require_device(mtg_ctx * ctx)
   if (!ctx)
     return MTG_ERR_BAD_INPUT;
   CK(cudaSetDevice(ctx->device));
+  return MTG_OK;
+}
+
+mtg_status
+quadrature_ready(mtg_ctx * ctx)
+{
+  if (!ctx->quad_ready)
+    CK(upload_quadrature());
+  ctx->quad_ready = true;
   return MTG_OK;
 }
 
@@ -1451,6 +1461,9 @@ mtg_surrogate_train(mtg_ctx * ctx, const mtg_surrogate_config * cfg, mtg_surroga
   CK(ensure(ctx->d_sg_params, 4 * MTG_SURROGATE_NPARAM));
   CK(ensure(ctx->d_sg_net, surrogate_net_bytes()));
   double loss = 0.0, secs = 0.0;
+  st = quadrature_ready(ctx);
+  if (st != MTG_OK)
+    return st;
   CK(surrogate_train(cfg->n_train, cfg->batch, cfg->epochs, cfg->qat_epochs, cfg->lr, cfg->seed, cfg->w_tau,
                      cfg->target, cfg->weighting, ptr<float>(ctx->d_sg_params), ctx->d_sg_net.p, &loss, &secs));
   ctx->sg_ready = true;
@@ -1530,6 +1543,9 @@ mtg_surrogate_quadrature(mtg_ctx * ctx, const double * eps, const double * b, lo
   CK(ensure(ctx->d_tmp3, 8 * size_t(n)));
   CK(cudaMemcpy(ctx->d_tmp0.p, eps, 8 * n, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ctx->d_tmp1.p, b, 8 * n, cudaMemcpyHostToDevice));
+  st = quadrature_ready(ctx);
+  if (st != MTG_OK)
+    return st;
   CK(launch_quadrature(ptr<double>(ctx->d_tmp0), ptr<double>(ctx->d_tmp1), n, ptr<double>(ctx->d_tmp2),
                        ptr<double>(ctx->d_tmp3), nullptr));
   CK(cudaMemcpy(s2, ctx->d_tmp2.p, 8 * n, cudaMemcpyDeviceToHost));

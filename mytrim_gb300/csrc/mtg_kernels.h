@@ -56,6 +56,7 @@ cudaError_t upload_newton_guess32();
 cudaError_t upload_newton_guess32_surrogate(const float * table);
 
 // Surrogate (mtg_surrogate.cu)
+cudaError_t upload_quadrature(); // the quadrature's tables, before launch_quadrature or surrogate_train
 cudaError_t launch_quadrature(const double * eps, const double * b, long long n, double * s2, double * tau,
                               cudaStream_t st);
 cudaError_t launch_surrogate_eval(const void * net, const double * eps, const double * b, long long n, double * s2,

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "mytrim_gpu.h"
@@ -676,55 +677,69 @@ surrogate_eval_kernel(const SurrogateNet * gnet, const double * eps, const doubl
 namespace mtg
 {
 
-// the quadrature's nodes and the pieces of phi, once per process
-static void
-upload_nodes_once()
+// the quadrature's nodes and the pieces of phi, made once per process
+struct QuadTables
 {
-  static bool done = false;
-  if (done)
-    return;
-  const double pi = 3.14159265358979323846;
   QuadNode nodes[QN / 2];
-  for (int j = 1; j <= QN / 2; ++j)
-  {
-    const double u = std::cos((2.0 * j - 1.0) * pi / (2.0 * QN));
-    const double s = std::sqrt(1.0 - u * u);
-    nodes[j - 1] = QuadNode{1.0 / u, u, u * u, s, s / (u * u)};
-  }
-  cudaMemcpyToSymbol(c_nodes, nodes, sizeof nodes);
-  // each piece: the interpolant at its PHI_N Chebyshev points, as a Chebyshev series
-  // c_0 / 2 + sum c_k T_k(t), then in powers of t
-  std::vector<double> table(size_t(PHI_OCT << PHI_BITS) * PHI_N);
-  double T[PHI_N][PHI_N] = {}; // T_k's coefficients
-  T[0][0] = T[1][1] = 1.0;
-  for (int k = 2; k < PHI_N; ++k)
-    for (int i = 0; i < PHI_N; ++i)
-      T[k][i] = (i > 0 ? 2.0 * T[k - 1][i - 1] : 0.0) - T[k - 2][i];
-  for (int p = 0; p < PHI_OCT << PHI_BITS; ++p)
-  {
-    const double a = std::ldexp(1.0 + double(p & ((1 << PHI_BITS) - 1)) / (1 << PHI_BITS), PHI_LO + (p >> PHI_BITS));
-    const double h = std::ldexp(1.0, PHI_LO + (p >> PHI_BITS) - PHI_BITS);
-    double y[PHI_N];
-    for (int m = 0; m < PHI_N; ++m)
-      y[m] = screening(a + 0.5 * h * (std::cos((2 * m + 1) * pi / (2 * PHI_N)) + 1.0));
-    for (int k = 0; k < PHI_N; ++k)
+  std::vector<double> phi;
+};
+
+static const QuadTables &
+quad_tables()
+{
+  static QuadTables q;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    const double pi = 3.14159265358979323846;
+    for (int j = 1; j <= QN / 2; ++j)
     {
-      double c = 0.0;
-      for (int m = 0; m < PHI_N; ++m)
-        c += y[m] * std::cos(k * (2 * m + 1) * pi / (2 * PHI_N));
-      c *= (k > 0 ? 2.0 : 1.0) / PHI_N;
-      for (int i = 0; i < PHI_N; ++i)
-        table[size_t(p) * PHI_N + i] += c * T[k][i];
+      const double u = std::cos((2.0 * j - 1.0) * pi / (2.0 * QN));
+      const double s = std::sqrt(1.0 - u * u);
+      q.nodes[j - 1] = QuadNode{1.0 / u, u, u * u, s, s / (u * u)};
     }
-  }
-  cudaMemcpyToSymbol(g_phi, table.data(), sizeof(double) * table.size());
-  done = true;
+    // each piece: the interpolant at its PHI_N Chebyshev points, as a Chebyshev series
+    // c_0 / 2 + sum c_k T_k(t), then in powers of t
+    q.phi.resize(size_t(PHI_OCT << PHI_BITS) * PHI_N);
+    double T[PHI_N][PHI_N] = {}; // T_k's coefficients
+    T[0][0] = T[1][1] = 1.0;
+    for (int k = 2; k < PHI_N; ++k)
+      for (int i = 0; i < PHI_N; ++i)
+        T[k][i] = (i > 0 ? 2.0 * T[k - 1][i - 1] : 0.0) - T[k - 2][i];
+    for (int p = 0; p < PHI_OCT << PHI_BITS; ++p)
+    {
+      const double a = std::ldexp(1.0 + double(p & ((1 << PHI_BITS) - 1)) / (1 << PHI_BITS), PHI_LO + (p >> PHI_BITS));
+      const double h = std::ldexp(1.0, PHI_LO + (p >> PHI_BITS) - PHI_BITS);
+      double y[PHI_N];
+      for (int m = 0; m < PHI_N; ++m)
+        y[m] = screening(a + 0.5 * h * (std::cos((2 * m + 1) * pi / (2 * PHI_N)) + 1.0));
+      for (int k = 0; k < PHI_N; ++k)
+      {
+        double c = 0.0;
+        for (int m = 0; m < PHI_N; ++m)
+          c += y[m] * std::cos(k * (2 * m + 1) * pi / (2 * PHI_N));
+        c *= (k > 0 ? 2.0 : 1.0) / PHI_N;
+        for (int i = 0; i < PHI_N; ++i)
+          q.phi[size_t(p) * PHI_N + i] += c * T[k][i];
+      }
+    }
+  });
+  return q;
+}
+
+// onto the current device, for every context that integrates (before its first use): a
+// flag for the process would leave a second device, or one that was reset, with zeros.
+// Contexts that share a device write the same bytes.
+cudaError_t
+upload_quadrature()
+{
+  const QuadTables & q = quad_tables();
+  const cudaError_t e = cudaMemcpyToSymbol(c_nodes, q.nodes, sizeof q.nodes);
+  return e != cudaSuccess ? e : cudaMemcpyToSymbol(g_phi, q.phi.data(), sizeof(double) * q.phi.size());
 }
 
 cudaError_t
 launch_quadrature(const double * eps, const double * b, long long n, double * s2, double * tau, cudaStream_t st)
 {
-  upload_nodes_once();
   if (n > 0)
     quadrature_kernel<<<(unsigned int)((n + 127) / 128), 128, 0, st>>>(eps, b, n, s2, tau);
   return cudaGetLastError();
@@ -862,7 +877,6 @@ surrogate_train(long long n_train, int batch, int epochs, int qat_epochs, float 
                 float w_tau, int target, int weighting, float * params_dev, void * net_dev, double * final_loss,
                 double * train_seconds)
 {
-  upload_nodes_once();
   TrainShape shape;
   cudaError_t e = train_shape(batch, shape);
   if (e)
