@@ -52,14 +52,20 @@ screening(double r)
          0.028171 * exp64(-0.20162 * r);
 }
 
-// phi(r) as a polynomial of degree 7 on each 64th of an octave from 2^-6 to 2^8: 128
+// phi(r) as a polynomial of degree 7 on each 128th of an octave from 2^-6 to 2^8: 128
 // nodes a sample, on a unit that runs FP64 at 2 lanes per SM and clock, where the four
-// exponentials take 63 operations and this 9.  Its error is that of the exponentials'
-// own arguments (median 1.4e-16 against 6.6e-16, worst 7e-13 beyond r = 128, where phi is
-// below 1e-12); above 2^8 phi < 2e-24 counts as 0, below 2^-6 the exponentials stand.
-// Samples of the training set: 131,072 targets 6.0 -> 1.7 ms.
-constexpr int PHI_OCT = 14, PHI_LO = -6, PHI_BITS = 6, PHI_N = 8;
+// exponentials take 63 operations and this 9.  It is good to 1.5e-15 up
+// to r = 128 and to 4e-15 above, as the exponentials of rounded products are.  Below 2^-6 the exponentials
+// stand, from 2^8 on the last one of them (the others are below 1e-20 of it).
+constexpr int PHI_OCT = 14, PHI_LO = -6, PHI_BITS = 7, PHI_N = 8;
 static __device__ double g_phi[(PHI_OCT << PHI_BITS) * PHI_N];
+
+// phi(r) outside the table
+__device__ __forceinline__ double
+phi_outside(double r)
+{
+  return r < 1.0 ? screening(r) : 0.028171 * exp64(-0.20162 * r);
+}
 
 // t in [-1, 1) and the first coefficient of r's piece; NULL outside the table
 __device__ __forceinline__ const double *
@@ -74,13 +80,14 @@ phi_piece(double r, double & t)
   return g_phi + k * PHI_N;
 }
 
+// far: whether phi counts beyond the table
 __device__ __forceinline__ double
-phi_table(double r)
+phi_table(double r, bool far)
 {
   double t;
   const double * c = phi_piece(r, t);
   if (!c)
-    return r < 1.0 ? screening(r) : 0.0;
+    return far || r < 1.0 ? phi_outside(r) : 0.0;
   double v = c[PHI_N - 1];
 #pragma unroll
   for (int i = PHI_N - 2; i >= 0; --i)
@@ -96,8 +103,8 @@ phi_slope(double r, double & phi, double & dphi)
   const double * c = phi_piece(r, t);
   if (!c)
   {
-    phi = r < 1.0 ? screening(r) : 0.0;
-    dphi = r < 1.0 ? -1.0 : 0.0; // within a factor of 1.3 of the slope below 2^-6
+    phi = phi_outside(r);
+    dphi = r < 1.0 ? -1.0 : -0.20162 * phi; // below 2^-6 within a factor of 1.3, for Newton steps
     return;
   }
   double v = c[PHI_N - 1], d = 0.0;
@@ -154,13 +161,16 @@ scatter_quadrature(double eps, double b, double & s2, double & tau)
   const double beta = b / r0;
   const double beta2 = beta * beta;
   const double ie = 1.0 / (r0 * eps);
+  // from r = 256 on phi u / (r0 eps) = phi / (r eps) is below 5e-27 / eps: less than half
+  // an ulp of h2 below, which r0 <= 64 keeps above 0.9 there
+  const bool far = !(eps >= 1e-9 && r0 <= 64.0);
   double I = 0.0, J = 0.0;
 #pragma unroll 2
   for (int j = 0; j < QN / 2; ++j)
   {
     const QuadNode & n = c_nodes[j];
     const double h2 = fma(-beta2, n.u2, 1.0);                           // 1 - beta^2 u^2
-    const double g2 = fma(-phi_table(r0 * n.inv_u), n.u * ie, h2);
+    const double g2 = fma(-phi_table(r0 * n.inv_u, far), n.u * ie, h2);
     const double ig = rsqrt(g2);
     I = fma(n.s, ig, I);
     J = fma(n.s_u2, ig - rsqrt(h2), J);
@@ -684,6 +694,20 @@ struct QuadTables
   std::vector<double> phi;
 };
 
+// phi(r) with the rounding of each exponent's product made good (host)
+static double
+screening_exact(double r)
+{
+  const double c[4] = {0.18175, 0.50986, 0.28022, 0.028171}, d[4] = {3.1998, 0.94229, 0.4029, 0.20162};
+  double phi = 0.0;
+  for (int i = 0; i < 4; ++i)
+  {
+    const double x = -d[i] * r, e = exp64(x);
+    phi += c[i] * fma(e, fma(-d[i], r, -x), e);
+  }
+  return phi;
+}
+
 static const QuadTables &
 quad_tables()
 {
@@ -711,7 +735,7 @@ quad_tables()
       const double h = std::ldexp(1.0, PHI_LO + (p >> PHI_BITS) - PHI_BITS);
       double y[PHI_N];
       for (int m = 0; m < PHI_N; ++m)
-        y[m] = screening(a + 0.5 * h * (std::cos((2 * m + 1) * pi / (2 * PHI_N)) + 1.0));
+        y[m] = screening_exact(a + 0.5 * h * (std::cos((2 * m + 1) * pi / (2 * PHI_N)) + 1.0));
       for (int k = 0; k < PHI_N; ++k)
       {
         double c = 0.0;
