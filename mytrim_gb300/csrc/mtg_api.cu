@@ -680,6 +680,7 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
   if (ctx->cfg.precision == MTG_PREC_FP32_SURROGATE && !ctx->sg_ready)
     return fail(ctx, MTG_ERR_STATE, "no trained surrogate: call mtg_surrogate_train or mtg_surrogate_set_params");
   std::string err;
+  ctx->prepared = ctx->launched = false; // the tables of the last run go now, also where these are refused
   int rc = build_tables(ctx->rows, ctx->cfg, sims, n_sims, ctx->tables, err);
   if (rc != MTG_OK)
     return fail(ctx, mtg_status(rc), err);
@@ -691,7 +692,6 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
   const bool voxels = t.voxel_total > 0;
 
   // the run's results first (collect copies them together), then what else a run clears
-  ctx->prepared = ctx->launched = false;
   CK(cut(ctx->d_run, {{&ctx->d_counters, 8 * C_COUNT},
                       {&ctx->d_err, 16},
                       {&ctx->d_totals, sizeof(SimTotals) * ns},
@@ -840,7 +840,6 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
     return st;
   CK(cudaDeviceSynchronize()); // the tables are in place for a launch on any stream
   ctx->prepared = true;
-  ctx->launched = false;
   return MTG_OK;
 }
 
