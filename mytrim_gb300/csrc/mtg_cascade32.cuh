@@ -648,6 +648,7 @@ again:
       top -= npop;
       if (avail <= need)
         work_done = true;
+      __syncwarp(); // popped before another lane pushes into the same place
       if (__ballot_sync(FULL, live) == 0)
         break;
     }

@@ -1139,6 +1139,7 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
     const unsigned int idle = __ballot_sync(FULL, !live);
     if (idle && __popc(idle) >= prm.refill_min)
     {
+      __syncwarp(); // the recoils other lanes pushed
       const int nidle = __popc(idle);
       const int rank = __popc(idle & lt);
       const int npop = nidle < top ? nidle : top;
@@ -1176,6 +1177,7 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
           live = true;
         }
       }
+      __syncwarp(); // popped before another lane pushes into the same place
     }
     if (__ballot_sync(FULL, live) == 0)
     {
