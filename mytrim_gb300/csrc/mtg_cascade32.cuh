@@ -436,6 +436,11 @@ cascade32_kernel(const __grid_constant__ EngineParams prm, const __grid_constant
   using Sink = LaneSink<Sink32, LVL>;
   using Rec = std::conditional_t<Sink::EV, Rec32Tag, Rec32>;
   extern __shared__ __align__(16) unsigned char smem[];
+  // recoils sent between warps: with the network only (Ag into Si, 50,000 primaries: 113 ->
+  // 99 ms; the exact kernels gain up to 7 % of some runs and lose up to 8 % of others)
+  constexpr bool SHARE = SURROGATE;
+  if constexpr (SHARE)
+    RecoilPool<Rec>::start(prm.pool);
 
   // per-block vacancy / replacement counters, material rows and the network
   unsigned int * s_hist = reinterpret_cast<unsigned int *>(smem + prm.hist_smem_offset);
@@ -501,9 +506,6 @@ cascade32_kernel(const __grid_constant__ EngineParams prm, const __grid_constant
   sink.reset_sim();
   sink.reset_member();
 
-  // recoils sent between warps: with the network only (Ag into Si, 50,000 primaries: 113 ->
-  // 99 ms; the exact kernels gain up to 7 % of some runs and lose up to 8 % of others)
-  constexpr bool SHARE = SURROGATE;
   [[maybe_unused]] RecoilPool<Rec> pool;
   [[maybe_unused]] bool give = false;
   unsigned int steps = 0;

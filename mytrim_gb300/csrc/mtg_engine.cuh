@@ -140,8 +140,11 @@ struct EngineParams
 //
 // Nothing here depends on another warp's progress but the last step of a letter, between
 // a sender's claim of a mailbox and its note that the recoils are in it.  An idle warp
-// leaves when all others are idle or gone, or after PATIENCE ns; it gives up its mailbox
-// first, by a compare-and-swap that fails if a sender has claimed it.
+// leaves when all others that have started are idle or gone, or after PATIENCE ns; it gives
+// up its mailbox first, by a compare-and-swap that fails if a sender has claimed it.  (A
+// grid need not be resident as a whole: another stream's kernel may hold a part of the
+// SMs.  An idle warp finds all work taken, by warps that have started, so those that have
+// not bring none.)
 //
 // FP64 kernel, Ag 200 keV into Si: 64 primaries 55 -> 42 ms, 1000 107 -> 87 ms, 2000
 // 153 -> 139 ms.  With the network, 50,000 Ag 113 -> 100 ms.  The exact FP32 kernel goes
@@ -150,7 +153,8 @@ struct EngineParams
 // and the 4096-simulation batch 12.
 struct PoolControl
 {
-  unsigned int hungry, gone; // warps waiting, warps that left
+  unsigned int hungry; // warps waiting
+  int active;          // warps that have started and neither wait nor left
   unsigned int pad0[30];
   int avail; // entries of the ring that no sender has taken
   unsigned int pad1[31];
@@ -176,6 +180,14 @@ struct RecoilPool
     return (prm.pool_nonce << 10) ^ (ticket >> RING_BITS);
   }
 
+  // a block's first step, before it takes work; a call, because inlined it moves the hot
+  // loop's registers (50,000 Ag with the network 100.9 -> 102.3 ms)
+  static __device__ __noinline__ void start(PoolControl * ctl)
+  {
+    if (threadIdx.x == 0)
+      atomicAdd(&ctl->active, int(blockDim.x >> 5));
+  }
+
   // an idle warp waits for recoils (all lanes) and puts them on its empty stack; their
   // number, 0: none will come
   static __device__ __forceinline__ int wait(const EngineParams & prm, unsigned int warp, Rec * stack, int lane)
@@ -186,11 +198,11 @@ struct RecoilPool
     if (lane == 0)
     {
       PoolControl * ctl = prm.pool;
-      const unsigned int warps = gridDim.x * (blockDim.x >> 5);
       unsigned int * box = prm.pool_box + warp;
       const volatile unsigned int * vbox = box;
       *reinterpret_cast<volatile unsigned int *>(box) = WAITING;
       atomicAdd(&ctl->hungry, 1u);
+      atomicSub(&ctl->active, 1);
       const unsigned int t = atomicAdd(&ctl->tail, 1u);
       asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(prm.pool_ring + (t & (RING - 1))),
                    "l"((unsigned long long)tag(prm, t) << 32 | (warp + 1u))
@@ -210,9 +222,10 @@ struct RecoilPool
         unsigned int ns = 200u;
         if (!claimed)
         {
-          unsigned int hungry, gone;
-          asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(hungry), "=r"(gone) : "l"(ctl) : "memory");
-          if (hungry + gone >= warps || slept >= PATIENCE)
+          unsigned int hungry;
+          int active;
+          asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(hungry), "=r"(active) : "l"(ctl) : "memory");
+          if (active <= 0 || slept >= PATIENCE)
           {
             if (atomicCAS(box, WAITING, LEFT) == WAITING)
               break;
@@ -227,11 +240,13 @@ struct RecoilPool
       {
         if (claimed)
           atomicOr(prm.error_flags, ERRB_QUEUE_FULL); // the sender never came: the run is made again
-        atomicAdd(&ctl->gone, 1u);
+      }
+      else
+      {
+        atomicAdd(&ctl->active, 1);
+        __threadfence(); // the letter's recoils after its note
       }
       atomicSub(&ctl->hungry, 1u);
-      if (k != 0u)
-        __threadfence(); // the letter's recoils after its note
     }
     k = __shfl_sync(0xffffffffu, k, 0);
     __syncwarp();
@@ -1031,6 +1046,7 @@ cascade_kernel(const EngineParams prm, const typename Pol::Tables tabs)
   extern __shared__ __align__(16) unsigned char smem[];
   if (prm.in_records && *prm.in_count == 0)
     return; // a drain pass with nothing to drain
+  RecoilPool<Particle>::start(prm.pool);
 
   // stage the tables of a single-simulation run in shared memory
   // per-block vacancy / replacement counters (zeroed before the staging barrier)
