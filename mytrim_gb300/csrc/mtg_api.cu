@@ -97,7 +97,6 @@ enum Counter
   C_COUNT = 72
 };
 constexpr int MAX_PASSES = 64;
-constexpr int MAX_OVF_RETRIES = 3; // runs redone with a larger overflow list
 
 } // namespace
 
@@ -905,7 +904,7 @@ grow_overflow(mtg_ctx * ctx, long long cap)
 }
 
 static mtg_status
-collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry);
+collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int attempt, int enlarged);
 
 mtg_status
 mtg_collect(mtg_ctx * ctx, mtg_totals * totals, long long * hist)
@@ -915,11 +914,11 @@ mtg_collect(mtg_ctx * ctx, mtg_totals * totals, long long * hist)
     return st;
   if (!ctx->launched)
     return fail(ctx, MTG_ERR_STATE, "nothing launched");
-  return collect_run(ctx, totals, hist, 0);
+  return collect_run(ctx, totals, hist, 0, 0);
 }
 
 static mtg_status
-collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
+collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int attempt, int enlarged)
 {
   mtg_status st = MTG_OK;
   const HostTables & t = ctx->tables;
@@ -956,15 +955,17 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
   // an overflow list that filled dropped members: the run is made again with lists
   // four times larger, kept for later runs.  The random draws depend on the members'
   // keys, not on the schedule, so the repeated run is the run the larger lists would
-  // have given in the first place.
-  if ((errf & ERRB_QUEUE_FULL) && retry < MAX_OVF_RETRIES && grow_overflow(ctx, ctx->ovf_cap * 4))
+  // have given in the first place.  So is a run that lost recoils between warps, with
+  // the lists as they are.
+  const Again again = make_again(errf, attempt);
+  if (again == Again::SAME || (again == Again::LARGER && grow_overflow(ctx, ctx->ovf_cap * 4)))
   {
     const int launched_before = ctx->stats.launches; // the count covers every attempt
     st = mtg_launch_async(ctx, ctx->stream);
     if (st != MTG_OK)
       return st;
     ctx->stats.launches += launched_before;
-    return collect_run(ctx, totals, hist, retry + 1);
+    return collect_run(ctx, totals, hist, attempt + 1, enlarged + (again == Again::LARGER));
   }
   if (extra)
   {
@@ -985,7 +986,7 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
   ctx->stats.kernel_ms = ms;
   cudaEventElapsedTime(&ms, extra ? ctx->ev[3] : ctx->ev[1], ctx->ev[2]);
   ctx->stats.reduce_ms = ms;
-  ctx->stats.overflow_retries = retry;
+  ctx->stats.overflow_retries = enlarged;
   ctx->stats.drains = ctx->passes - 1;
   ctx->stats.warp_steps = (long long)cnt[C_STEPS];
   ctx->stats.grid = ctx->grid;
@@ -1049,6 +1050,8 @@ collect_run(mtg_ctx * ctx, mtg_totals * totals, long long * hist, int retry)
   // a full event log is reported last: any other error of the run takes precedence
   if (unfinished || (errf & ERRB_QUEUE_FULL))
     return fail(ctx, MTG_ERR_QUEUE_FULL, "recoil overflow list exhausted; results incomplete");
+  if (errf & ERRB_LOST_LETTER)
+    return fail(ctx, MTG_ERR_CUDA, "recoils sent between warps did not arrive in time; results incomplete");
   if (errf & ERRB_BUDGET)
     return fail(ctx, MTG_ERR_TIMEOUT, "a cascade member exceeded the collision budget");
   if (errf & ERRB_NUMERIC)

@@ -12,7 +12,8 @@
 //   * recoils are pushed with a ballot + prefix count; a full stack spills into
 //     a global overflow list that a follow-up launch drains.
 // In the FP64 and surrogate kernels a busy warp sends recoils to warps that have run
-// out (RecoilPool); the only wait in them is an idle warp's, for 20 ms at most.  Every
+// out (RecoilPool); the only wait in them is an idle warp's, for 20 ms of sleep and, for
+// recoils already on their way to it, another 20 at most.  Every
 // loop is bounded (collisions per member, Newton iterations, rejection passes).  The
 // single-precision kernel is in mtg_cascade32.cuh; it shares the tallies and parameters.
 //
@@ -129,7 +130,7 @@ struct EngineParams
 // A warp owns the cascades it started, and at the end of a run, or in a run of fewer
 // primaries than warps, most warps have none left while a few still have hundreds of
 // recoils on their stacks.  An idle warp enters its number in a ring and watches its own
-// mailbox; a busy warp looks every eighth iteration how many wait (at the count it loaded
+// mailbox; a busy warp looks every eighth iteration (FP64: every fourth) how many wait (at the count it loaded
 // the time before, so that it does not wait for it) and, while any do, sends one of them
 // the older half of its stack, 32 recoils at most, if they hold enough energy to be worth
 // the move (share_min): a mailbox per warp, because a common list of chunks that all idle
@@ -141,10 +142,11 @@ struct EngineParams
 // Nothing here depends on another warp's progress but the last step of a letter, between
 // a sender's claim of a mailbox and its note that the recoils are in it.  An idle warp
 // leaves when all others that have started are idle or gone, or after PATIENCE ns; it gives
-// up its mailbox first, by a compare-and-swap that fails if a sender has claimed it.  (A
-// grid need not be resident as a whole: another stream's kernel may hold a part of the
-// SMs.  An idle warp finds all work taken, by warps that have started, so those that have
-// not bring none.)
+// up its mailbox first, by a compare-and-swap that fails if a sender has claimed it.  Then
+// it waits for that letter, PATIENCE ns more at most (ERRB_LOST_LETTER: the run is made
+// again).  (A grid need not be resident as a whole: another stream's kernel may hold a
+// part of the SMs.  An idle warp finds all work taken, by warps that have started, so those
+// that have not bring none.)
 //
 // FP64 kernel, Ag 200 keV into Si: 64 primaries 55 -> 42 ms, 1000 107 -> 87 ms, 2000
 // 153 -> 139 ms.  With the network, 50,000 Ag 113 -> 100 ms.  The exact FP32 kernel goes
@@ -209,7 +211,7 @@ struct RecoilPool
                    : "memory");
       int before;
       asm volatile("atom.add.release.gpu.global.s32 %0, [%1], 1;" : "=r"(before) : "l"(&ctl->avail) : "memory");
-      unsigned int slept = 0;
+      unsigned int slept = 0, limit = PATIENCE;
       bool claimed = false;
       for (int i = 0; i < (1 << 20); ++i)
       {
@@ -225,21 +227,24 @@ struct RecoilPool
           unsigned int hungry;
           int active;
           asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(hungry), "=r"(active) : "l"(ctl) : "memory");
-          if (active <= 0 || slept >= PATIENCE)
+          if (active <= 0 || slept >= limit)
           {
             if (atomicCAS(box, WAITING, LEFT) == WAITING)
               break;
             claimed = true; // a sender is about to fill it
+            limit = slept + PATIENCE;
           }
           ns = min(max(500u, hungry * 2u), 10000u);
         }
+        else if (slept >= limit)
+          break;
         __nanosleep(ns);
         slept += ns;
       }
       if (k == 0u)
       {
         if (claimed)
-          atomicOr(prm.error_flags, ERRB_QUEUE_FULL); // the sender never came: the run is made again
+          atomicOr(prm.error_flags, ERRB_LOST_LETTER);
       }
       else
       {

@@ -16,6 +16,16 @@
 namespace mtg
 {
 
+Again
+make_again(unsigned int errors, int attempt)
+{
+  if (attempt >= MAX_ATTEMPTS)
+    return Again::NO;
+  if (errors & ERRB_QUEUE_FULL)
+    return Again::LARGER;
+  return errors & ERRB_LOST_LETTER ? Again::SAME : Again::NO;
+}
+
 void
 seed_key(unsigned long long seed, uint32_t & k0, uint32_t & k1)
 {

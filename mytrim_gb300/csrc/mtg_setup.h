@@ -62,6 +62,18 @@ int make_material(const mtg_scoef_row * rows, const SpeciesConst & sc, const mtg
 void build_fp32_tables(const HostTables & t, std::vector<Mat32> & mats, std::vector<MatCold32> & cold,
                        std::vector<Sim32> & sims);
 
+// Whether a run whose kernels set `errors` (ErrorBits) is made again, the `attempt`th time
+// (0 the first): with larger overflow lists where one filled, and as it was where recoils
+// were lost between warps.
+enum class Again
+{
+  NO,
+  SAME,
+  LARGER
+};
+constexpr int MAX_ATTEMPTS = 3;
+Again make_again(unsigned int errors, int attempt);
+
 // Philox key of a run seed
 void seed_key(unsigned long long seed, uint32_t & k0, uint32_t & k1);
 

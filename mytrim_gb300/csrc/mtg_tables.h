@@ -288,7 +288,8 @@ enum ErrorBits : unsigned int
   ERRB_NUMERIC = 2u,
   ERRB_BUDGET = 4u,
   ERRB_BAD_INDEX = 8u,
-  ERRB_EVENTS_FULL = 16u
+  ERRB_EVENTS_FULL = 16u,
+  ERRB_LOST_LETTER = 32u // recoils on their way between two warps did not arrive in time
 };
 
 } // namespace mtg

@@ -14,6 +14,7 @@
 // Checks of single pieces of the same code, for the tests:
 //   replay_host <tables> --stopping              "Z1 m1 rho n Z m t ...", then energies -> stopping (hex)
 //   replay_host <tables> --scatter [potential]   lines "eps b" -> sin^2(theta/2) (hex)
+//   replay_host <tables> --rules                the host's decisions about a launch (see there)
 //   replay_host <tables> --stopspecial          stopping at infinities, zeros, NaN: where it differs
 //   replay_host <tables> --mathcheck [n]         exp64 / log64 short routes vs full forms
 //   replay_host <tables> --eval exp|log|pow       lines of hex-float arguments -> results (hex)
@@ -242,6 +243,21 @@ main(int argc, char ** argv)
     }
     printf("%lld %lld\n", checked, bad);
     return bad ? 1 : 0;
+  }
+  if (argc >= 3 && std::string(argv[2]) == "--rules")
+  {
+    // decisions of the host about a launch, one per line:
+    //   again <error bits> <attempt>     0 no, 1 as it was, 2 with larger lists
+    std::string what;
+    while (std::cin >> what)
+      if (what == "again")
+      {
+        unsigned int errors;
+        int attempt;
+        std::cin >> errors >> attempt;
+        printf("%d\n", int(make_again(errors, attempt)));
+      }
+    return 0;
   }
   if (argc >= 3 && std::string(argv[2]) == "--stopspecial")
   {
