@@ -144,6 +144,7 @@ struct mtg_ctx
   int stage = 0;
   int stack_cap = 0;
   long long ovf_cap = 0;
+  long long trial_of = 0;  // primaries of the run that a tuning trial stands for, else 0
   long long ovf_floor = 0; // smallest overflow list of later runs, raised when a run exhausted one
   long long record_cap = 0;
   long long event_cap = 0;
@@ -444,30 +445,12 @@ launch_pass(mtg_ctx * ctx, int pass)
 
   cudaError_t e;
   const int prec = ctx->cfg.precision;
-  // A warp's lanes idle until its first cascades branch: without a pace it takes about 8
-  // primaries at once, and those that a run has beyond that are started last and end last.
-  // In runs of one simulation with 12 to 64 primaries per warp, a warp that has members
-  // takes one in every 8 or 16 iterations, which is a sixteenth or less of what an average
-  // one needs (about 11 collisions per member over 32 lanes); not where the cascades are
-  // small or cut short (by a generation limit, a high Ef or a box of less than 1 A per keV
-  // along a CUT axis).  FP32 kernel, ms without and with, by primaries per warp:
-  //                   10               12              20              60              120
-  //   Ag 200 keV  32.8 -> 28.5    38.7 -> 33.0    57.0 -> 52.3  151.6 -> 147.9  290.5 -> 290.6
-  //   Cu 100 keV  16.1 -> 15.6    20.3 -> 18.2    31.8 -> 28.8    82.2 -> 81.1  158.5 -> 159.1
-  //   As 50 keV   10.3 -> 10.8    14.3 -> 12.5    21.9 -> 19.7    55.4 -> 55.2  106.5 -> 108.7
-  //   Au 1 MeV     189 -> 171      232 -> 198      354 -> 312
-  // (Ag 200 keV with 8 per warp: 21.1 -> 22.7).
-  prm.take_mask = 0;
-  const long long share = prm.total_primaries / ((long long)ctx->grid * (ctx->block / 32));
-  if (pass == 0 && prec == MTG_PREC_FP32 && prm.stage_tables && share >= 12 && share < 64)
-  {
-    const SimDesc & d = ctx->tables.sims[0];
-    bool whole = !ctx->tables.any_mode && d.Ef <= 50.0;
-    for (int k = 0; k < 3; ++k)
-      whole = whole && (d.bc[k] != 2 || d.w[k] * ctx->cfg.length_scale >= 1e-3 * d.E0);
-    const double m = whole ? ctx->tables.members_est / 32.0 : 0.0;
-    prm.take_mask = m >= 16.0 ? 15u : m >= 8.0 ? 7u : 0u;
-  }
+  // a tuning trial is launched as the run that it stands for
+  const long long primaries = ctx->trial_of > 0 ? ctx->trial_of : prm.total_primaries;
+  prm.take_mask =
+      pass == 0 && prm.stage_tables
+          ? pace_mask(ctx->tables, ctx->cfg, primaries, (long long)ctx->grid * (ctx->block / 32))
+          : 0u;
   // No more blocks than have a primary for each warp, and as many on each SM: the resident
   // blocks of a full grid come to the counter SM by SM, and some SMs' warps take all there is
   // while others take none (FP32, 3000 Au 1 MeV: 16.7 -> 11.8 ms, 2500 Ag 200 keV: 2.93 ->
@@ -477,7 +460,7 @@ launch_pass(mtg_ctx * ctx, int pass)
   if (pass == 0 && (prec == MTG_PREC_FP32 || prm.share_after == RecoilPool<int>::NO_SHARING))
   {
     const long long per_wave = (long long)ctx->n_sm * (ctx->block / 32);
-    const long long waves = std::max<long long>(1, (prm.total_primaries + per_wave - 1) / per_wave);
+    const long long waves = std::max<long long>(1, (primaries + per_wave - 1) / per_wave);
     grid = int(std::min<long long>(grid, ctx->n_sm * waves));
   }
   if (prec == MTG_PREC_FP64)
@@ -1099,6 +1082,13 @@ mtg_autotune(mtg_ctx * ctx, const mtg_sim * sims, int n_sims, long long trial_pr
     if (s.n_primaries > 0)
       s.n_primaries = std::max<long long>(1, llround(double(s.n_primaries) * f));
   const mtg_config base = ctx->cfg;
+  // the trials' kernels and grids are the run's, whatever their own number of primaries
+  struct Trial
+  {
+    mtg_ctx * ctx;
+    ~Trial() { ctx->trial_of = 0; }
+  } of{ctx};
+  ctx->trial_of = total;
   std::vector<mtg_totals> tot(static_cast<size_t>(n_sims));
   int trials = 0;
   struct Setting

@@ -16,6 +16,35 @@
 namespace mtg
 {
 
+// A warp's lanes idle until its first cascades branch: without a pace it takes about 8
+// primaries at once, and those that a run has beyond that are started last and end last.
+// In FP32 runs of one simulation with 12 to 64 primaries per warp, a warp that has members
+// takes one in every 8 or 16 iterations, which is a sixteenth or less of what an average
+// one needs (about 11 collisions per member over 32 lanes); not where the cascades are
+// small or cut short (by a generation limit, a high Ef or a box of less than 1 A per keV
+// along a CUT axis).  Kernel ms without and with, by primaries per warp:
+//                   10               12              20              60              120
+//   Ag 200 keV  32.8 -> 28.5    38.7 -> 33.0    57.0 -> 52.3  151.6 -> 147.9  290.5 -> 290.6
+//   Cu 100 keV  16.1 -> 15.6    20.3 -> 18.2    31.8 -> 28.8    82.2 -> 81.1  158.5 -> 159.1
+//   As 50 keV   10.3 -> 10.8    14.3 -> 12.5    21.9 -> 19.7    55.4 -> 55.2  106.5 -> 108.7
+//   Au 1 MeV     189 -> 171      232 -> 198      354 -> 312
+// (Ag 200 keV with 8 per warp: 21.1 -> 22.7).  Also where the caller says how many a warp
+// takes at once: 20 per warp of Ag 200 keV, 1 at once 58.8 -> 51.7, 4 59.1 -> 55.1, 32
+// 87.3 -> 88.1; As 50 keV 1 18.3 -> 16.6, 4 18.9 -> 18.3, 32 27.1 -> 27.1.
+unsigned int
+pace_mask(const HostTables & t, const mtg_config & cfg, long long primaries, long long warps)
+{
+  const long long share = primaries / std::max<long long>(1, warps);
+  if (cfg.precision != MTG_PREC_FP32 || t.sims.size() != 1 || share < 12 || share >= 64)
+    return 0u;
+  const SimDesc & d = t.sims[0];
+  bool whole = !t.any_mode && d.Ef <= 50.0;
+  for (int k = 0; k < 3; ++k)
+    whole = whole && (d.bc[k] != 2 || d.w[k] * cfg.length_scale >= 1e-3 * d.E0);
+  const double m = whole ? t.members_est / 32.0 : 0.0;
+  return m >= 16.0 ? 15u : m >= 8.0 ? 7u : 0u;
+}
+
 Again
 make_again(unsigned int errors, int attempt)
 {

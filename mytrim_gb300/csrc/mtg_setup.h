@@ -62,6 +62,9 @@ int make_material(const mtg_scoef_row * rows, const SpeciesConst & sc, const mtg
 void build_fp32_tables(const HostTables & t, std::vector<Mat32> & mats, std::vector<MatCold32> & cold,
                        std::vector<Sim32> & sims);
 
+// EngineParams::take_mask of a launch of `primaries` on `warps` warps.
+unsigned int pace_mask(const HostTables & t, const mtg_config & cfg, long long primaries, long long warps);
+
 // Whether a run whose kernels set `errors` (ErrorBits) is made again, the `attempt`th time
 // (0 the first): with larger overflow lists where one filled, and as it was where recoils
 // were lost between warps.

@@ -248,6 +248,8 @@ main(int argc, char ** argv)
   {
     // decisions of the host about a launch, one per line:
     //   again <error bits> <attempt>     0 no, 1 as it was, 2 with larger lists
+    //   pace <precision> <primaries> <warps> <simulations> <members>
+    //                                    iterations between two refills with new work, less one
     std::string what;
     while (std::cin >> what)
       if (what == "again")
@@ -256,6 +258,19 @@ main(int argc, char ** argv)
         int attempt;
         std::cin >> errors >> attempt;
         printf("%d\n", int(make_again(errors, attempt)));
+      }
+      else if (what == "pace")
+      {
+        mtg_config cfg;
+        memset(&cfg, 0, sizeof cfg);
+        cfg.length_scale = 1.0;
+        HostTables t;
+        long long primaries, warps;
+        int sims;
+        std::cin >> cfg.precision >> primaries >> warps >> sims >> t.members_est;
+        t.sims.resize(size_t(sims));
+        t.sims[0].Ef = 5.0;
+        printf("%u\n", pace_mask(t, cfg, primaries, warps));
       }
     return 0;
   }
