@@ -793,8 +793,16 @@ surrogate_net_bytes()
 }
 
 // A training pass's tile and blocks: one block per SM of the current device at most, and
-// the tile that leaves the fewest samples to the block with the most (16,384 samples on
-// 152 SMs: two tiles of 56 instead of two of 64, 42.9 -> 41 us a pass; 4096: one of 28).
+// the tile whose busiest block is done first.  A tile of TS samples takes a time like
+// TS + TILE_FIXED: measured 15, 14 and 8.5 us for 64, 56 and 28 (the threads of the 64 x 64
+// products that a small tile leaves idle take as long as the others, and so do the
+// barriers).  us per step, Adam's included, by batch, for tiles of 64, 56 and 28:
+//     4096  28.9  30.7  28.0      12000  47.7  45.4  44.7      26000  62.7  71.7  76.9
+//     8192  31.1  33.0  36.1      16384  48.4  46.3  53.0      29185  75.9  72.1  77.9
+//     9000  31.2  45.2  43.5      20000  61.6  59.5  61.5      32768  77.1  72.3  86.4
+//    10007  47.0  45.4  44.5      25536  62.9  59.5  70.0      65536 120.8 125.6 152.4
+// (by samples alone 20,000 and 29,185 went to 28.)
+constexpr int TILE_FIXED = 19;
 struct TrainShape
 {
   void (*kernel)(const float *, const float *, const float *, long long, long long, const int *, const float *, int,
@@ -808,10 +816,10 @@ static void
 try_tile(long long B, int sms, long long & best, TrainShape & t)
 {
   const long long tiles = (B + TS - 1) / TS;
-  const long long rows = (tiles + sms - 1) / sms * TS;
-  if (t.kernel && rows >= best)
+  const long long time = (tiles + sms - 1) / sms * (TS + TILE_FIXED);
+  if (t.kernel && time >= best)
     return;
-  best = rows;
+  best = time;
   t.kernel = train_pass_kernel<TS>;
   t.blocks = int(std::min<long long>(tiles, sms));
   t.smem = sizeof(TrainSmem<TS>);
