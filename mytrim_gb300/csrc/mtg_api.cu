@@ -121,7 +121,7 @@ struct mtg_ctx
   std::vector<char> staging; // the tables on their way to d_tables
   char * h_results = nullptr; // pinned: counters, error flags, totals, sums and voxel sums of a run
   size_t h_bytes = 0, results_bytes = 0;
-  DevBuf d_sims, d_order, d_order_end, d_species, d_mats, d_row_species, d_stop;
+  DevBuf d_sims, d_order, d_order_end, d_species, d_mats, d_stop;
   DevBuf d_mats32, d_cold32, d_sims32;
   DevBuf d_sg_params, d_sg_net; // surrogate network
   DevBuf d_vox, d_vox_range, d_vox_sum, d_vox_part; // energy-deposition voxels
@@ -810,8 +810,8 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
     // FP32 path: stopping tables evaluated on the device in FP64, one row per
     // distinct (species, material) of the run
     const double lo = std::log(STOP_EMIN), hi = std::log(t.emax * 1.05);
-    CK(launch_build_stop_tables(ptr<SpeciesConst>(ctx->d_species), ptr<MatConst>(ctx->d_mats), nullptr, int(nrows),
-                                nullptr, ptr<float>(ctx->d_stop), lo, (hi - lo) / (STOP_N - 1), nullptr));
+    CK(launch_build_stop_tables(ptr<SpeciesConst>(ctx->d_species), ptr<MatConst>(ctx->d_mats), int(nrows),
+                                ptr<float>(ctx->d_stop), lo, (hi - lo) / (STOP_N - 1), nullptr));
   }
   if (ctx->record_cap > 0)
     CK(ensure(ctx->d_records, sizeof(MemberRecord) * size_t(ctx->record_cap)));
@@ -1385,11 +1385,8 @@ mtg_stopping(mtg_ctx * ctx, int Z1, double m1, const mtg_material * material, co
       emax = std::max(emax, E[i]);
     const double lo = std::log(STOP_EMIN), hi = std::log(std::max(emax, 1.0) * 1.05);
     const double dl = (hi - lo) / (STOP_N - 1);
-    CK(ensure(ctx->d_tmp3, 2 * sizeof(float) * STOP_N + sizeof(int)));
-    int zero = 0;
-    int * d_rs = reinterpret_cast<int *>(reinterpret_cast<char *>(ctx->d_tmp3.p) + 2 * sizeof(float) * STOP_N);
-    CK(cudaMemcpy(d_rs, &zero, sizeof zero, cudaMemcpyHostToDevice));
-    CK(launch_build_stop_tables(d_sc, d_mc, nullptr, 1, d_rs, ptr<float>(ctx->d_tmp3), lo, dl, nullptr));
+    CK(ensure(ctx->d_tmp3, 2 * sizeof(float) * STOP_N));
+    CK(launch_build_stop_tables(d_sc, d_mc, 1, ptr<float>(ctx->d_tmp3), lo, dl, nullptr));
     CK(launch_stopping32(ptr<float>(ctx->d_tmp3), float(lo), float(1.0 / dl), ptr<double>(ctx->d_tmp1), n,
                          ptr<double>(ctx->d_tmp2), nullptr));
   }

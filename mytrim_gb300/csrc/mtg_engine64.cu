@@ -218,8 +218,8 @@ namespace mtg
 // in ln E, the pair S(E) (the FP64 stopping above) and p_max(E), the maximum impact
 // parameter of the free flight (trim.C:88-94, the FP64 formula of collide64).
 __global__ void
-build_stop_tables_kernel(const SpeciesConst * species, const MatConst * mats, const int * row_mat, int n_rows,
-                         const int * row_species, float * out, double lnE_min, double dlnE)
+build_stop_tables_kernel(const SpeciesConst * species, const MatConst * mats, int n_rows, float * out, double lnE_min,
+                         double dlnE)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)n_rows * STOP_N)
@@ -227,22 +227,22 @@ build_stop_tables_kernel(const SpeciesConst * species, const MatConst * mats, co
   const int row = int(i / STOP_N);
   const int j = int(i % STOP_N);
   const double E = exp64(lnE_min + dlnE * double(j));
-  const MatConst & mc = mats[row_mat ? row_mat[row] : row];
+  const MatConst & mc = mats[row];
   const double eeg = sqrt(E * mc.f * mc.epsdg);
   const double pmax = mc.a / (eeg + sqrt(eeg) + 0.125 * pow64(eeg, 0.1));
-  out[2 * i] = float(material_stop64(species[row_species ? row_species[row] : row], mc, E));
+  out[2 * i] = float(material_stop64(species[row], mc, E));
   out[2 * i + 1] = float(pmax);
 }
 
 cudaError_t
-launch_build_stop_tables(const SpeciesConst * species, const MatConst * mats, const int * row_mat, int n_rows,
-                         const int * row_species, float * out, double lnE_min, double dlnE, cudaStream_t st)
+launch_build_stop_tables(const SpeciesConst * species, const MatConst * mats, int n_rows, float * out, double lnE_min,
+                         double dlnE, cudaStream_t st)
 {
   const long long n = (long long)n_rows * STOP_N;
   const int block = 256;
   if (n > 0)
-    build_stop_tables_kernel<<<(unsigned int)((n + block - 1) / block), block, 0, st>>>(
-        species, mats, row_mat, n_rows, row_species, out, lnE_min, dlnE);
+    build_stop_tables_kernel<<<(unsigned int)((n + block - 1) / block), block, 0, st>>>(species, mats, n_rows, out,
+                                                                                         lnE_min, dlnE);
   return cudaGetLastError();
 }
 

@@ -37,9 +37,9 @@ struct Fp32Tables
   const Sim32 * one_sim;  // host copies of a single-simulation run's constants, its device
   const SimDesc * one_desc; // pointers patched in
 };
-cudaError_t launch_build_stop_tables(const SpeciesConst * species, const MatConst * mats, const int * row_mat,
-                                     int n_rows, const int * row_species, float * out, double lnE_min,
-                                     double dlnE, cudaStream_t st);
+// one row per species[r], mats[r]
+cudaError_t launch_build_stop_tables(const SpeciesConst * species, const MatConst * mats, int n_rows, float * out,
+                                     double lnE_min, double dlnE, cudaStream_t st);
 cudaError_t launch_cascade32(const EngineParams & prm, const Fp32Tables & t, int grid, int block, size_t smem,
                              cudaStream_t st, int surrogate);
 cudaError_t occupancy32(int block, size_t smem, int * blocks_per_sm, int surrogate, int level, int one);
