@@ -56,10 +56,9 @@ proton_stop64_above(const StopPair & sp, double pe, double lpe)
 MTG_HD double
 proton_stop64(const StopPair & sp, double e)
 {
-  if (e <= 25.0)
-    return sp.s25 * pow64(e / 25.0, sp.velpwr);
-  const double pe = e > 25.0 ? e : 25.0; // an e that is not a number counts as 25
-  return proton_stop64_above(sp, pe, log64(pe));
+  if (e > 25.0)
+    return proton_stop64_above(sp, e, log64(e));
+  return e <= 25.0 ? sp.s25 * pow64(e / 25.0, sp.velpwr) : sp.s25; // an e that is not a number counts as 25
 }
 
 // relative velocity of a heavy ion over its Z1^(2/3), before the cut at yrcut
