@@ -195,9 +195,10 @@ typedef struct
   int block_threads;     /* threads per block of the cascade kernel: 64 or 128, 0 = 128 */
   int max_primaries_per_refill; /* fresh primaries one warp takes at a time, 1..32;
                                    0 = chosen from the expected cascade size (one for
-                                   large cascades), the batch size and the grid.  FP32 runs of one
-                                   simulation with 12 to 64 primaries per warp take
-                                   them at a pace: in every 8th or 16th iteration */
+                                   large cascades), the batch size and the grid.  FP32
+                                   runs of one simulation with 12 to 64 primaries per
+                                   warp take them at a pace: in every 8th or 16th
+                                   iteration */
   int refill_min_idle;   /* lanes of a warp that must be idle before the warp gives them
                             new members (recoils from its stack, fresh primaries), 1..32;
                             waiting lets the member-start code run for several lanes at
@@ -431,9 +432,8 @@ typedef struct
  * overflow list) is skipped, and so is one whose trial spilled members to the
  * overflow list at a rate that, over the run's full primaries, would fill a quarter
  * of it.  The trials take the kernel variant and grid of the full run, and use the
- * context like ordinary runs (their
- * results are discarded).  No counterpart in the reference, whose threads take
- * primaries one at a time (apps/runmytrim.C:71-93). */
+ * context like ordinary runs (their results are discarded).  No counterpart in the
+ * reference, whose threads take primaries one at a time (apps/runmytrim.C:71-93). */
 mtg_status mtg_autotune(mtg_ctx * ctx, const mtg_sim * sims, int n_sims, long long trial_primaries,
                         mtg_tuning * out);
 

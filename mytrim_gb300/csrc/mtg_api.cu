@@ -115,6 +115,7 @@ struct mtg_ctx
   std::vector<Sim32> sm32;
   bool prepared = false;
   bool launched = false;
+  bool refused = false; // a prepare has cleared the tables of the launched run and made none
   // device buffers: d_tables and d_run are allocations, the next two lines and the primaries'
   // tallies, totals, histograms, error flags, counters and results are cut from them
   DevBuf d_tables, d_run;
@@ -662,10 +663,14 @@ mtg_prepare(mtg_ctx * ctx, const mtg_sim * sims, int n_sims)
   if (ctx->cfg.precision == MTG_PREC_FP32_SURROGATE && !ctx->sg_ready)
     return fail(ctx, MTG_ERR_STATE, "no trained surrogate: call mtg_surrogate_train or mtg_surrogate_set_params");
   std::string err;
-  ctx->prepared = ctx->launched = false; // the tables of the last run go now, also where these are refused
+  // the tables of the last run go now, also where these simulations are refused; its
+  // events and member records can still be read then
+  ctx->prepared = false;
+  ctx->refused = true;
   int rc = build_tables(ctx->rows, ctx->cfg, sims, n_sims, ctx->tables, err);
   if (rc != MTG_OK)
     return fail(ctx, mtg_status(rc), err);
+  ctx->launched = ctx->refused = false;
   const HostTables & t = ctx->tables;
   const size_t ns = t.sims.size();
   const size_t np = size_t(std::max<long long>(t.total_primaries, 1));
@@ -895,7 +900,7 @@ mtg_collect(mtg_ctx * ctx, mtg_totals * totals, long long * hist)
   mtg_status st = require_device(ctx);
   if (st != MTG_OK)
     return st;
-  if (!ctx->launched)
+  if (!ctx->launched || ctx->refused)
     return fail(ctx, MTG_ERR_STATE, "nothing launched");
   return collect_run(ctx, totals, hist, 0, 0);
 }

@@ -13,9 +13,9 @@
 //     a global overflow list that a follow-up launch drains.
 // In the FP64 and surrogate kernels a busy warp sends recoils to warps that have run
 // out (RecoilPool); the only wait in them is an idle warp's, for 20 ms of sleep and, for
-// recoils already on their way to it, another 20 at most.  Every
-// loop is bounded (collisions per member, Newton iterations, rejection passes).  The
-// single-precision kernel is in mtg_cascade32.cuh; it shares the tallies and parameters.
+// recoils already on their way to it, another 20 at most.  Every loop is bounded
+// (collisions per member, Newton iterations, rejection passes).  The single-precision
+// kernel is in mtg_cascade32.cuh; it shares the tallies and parameters.
 //
 // Random numbers are keyed by the member's path key and collision index, so the
 // result does not depend on which lane or warp ran which member.
@@ -130,11 +130,12 @@ struct EngineParams
 // A warp owns the cascades it started, and at the end of a run, or in a run of fewer
 // primaries than warps, most warps have none left while a few still have hundreds of
 // recoils on their stacks.  An idle warp enters its number in a ring and watches its own
-// mailbox; a busy warp looks every eighth iteration (FP64: every fourth) how many wait (at the count it loaded
-// the time before, so that it does not wait for it) and, while any do, sends one of them
-// the older half of its stack, 32 recoils at most, if they hold enough energy to be worth
-// the move (share_min): a mailbox per warp, because a common list of chunks that all idle
-// warps watched was slower by a factor of a hundred than no sharing at all.
+// mailbox; a busy warp looks every eighth iteration (FP64: every fourth) how many wait (at
+// the count it loaded the time before, so that it does not wait for it) and, while any do,
+// sends one of them the older half of its stack, 32 recoils at most, if they hold enough
+// energy to be worth the move (share_min): a mailbox per warp, because a common list of
+// chunks that all idle warps watched was slower by a factor of a hundred than no sharing
+// at all.
 //
 // The notes are single releasing stores: a fence (__threadfence) also empties the SM's L1,
 // from which all its warps read their tables, and is left to the receipt of a letter.
