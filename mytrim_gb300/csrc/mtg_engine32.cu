@@ -95,7 +95,7 @@ occupancy32(int block, size_t smem, int * blocks_per_sm, int surrogate, int leve
   auto query = [&](auto * kernel) {
     if (smem > 48 * 1024)
     {
-      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      const cudaError_t e = allow_shared_memory(kernel);
       if (e != cudaSuccess)
         return e;
     }

@@ -121,11 +121,11 @@ launch_cascade64(const EngineParams & prm, int grid, int block, size_t smem, cud
 
 template <class K>
 static cudaError_t
-occupancy_of(K kernel, int block, size_t smem, int * blocks_per_sm)
+occupancy_of(K * kernel, int block, size_t smem, int * blocks_per_sm)
 {
   if (smem > 48 * 1024)
   {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const cudaError_t e = allow_shared_memory(kernel);
     if (e != cudaSuccess)
       return e;
   }

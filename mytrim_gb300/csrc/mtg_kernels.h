@@ -37,6 +37,21 @@ struct Fp32Tables
   const Sim32 * one_sim;  // host copies of a single-simulation run's constants, its device
   const SimDesc * one_desc; // pointers patched in
 };
+// The kernel's dynamic shared memory up to the device's limit, for all contexts: set to a
+// run's own size, the run of another context that needs less would take it away between
+// this one's prepare and its launch.
+template <class K>
+inline cudaError_t
+allow_shared_memory(K * kernel)
+{
+  int device = 0, most = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&device);
+  e = e ? e : cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  e = e ? e : cudaFuncGetAttributes(&a, kernel);
+  return e ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      most - int(a.sharedSizeBytes));
+}
 // one row per species[r], mats[r]
 cudaError_t launch_build_stop_tables(const SpeciesConst * species, const MatConst * mats, int n_rows, float * out,
                                      double lnE_min, double dlnE, cudaStream_t st);
